@@ -5,7 +5,9 @@
 //              the reference CPU hydro (src/hydro_utils.c) so that, compiled with
 //              -fmad=false and IEEE division/square root, results match the
 //              reference to the last bit except where libm pow() differs from
-//              CUDA's pow() (TRRS branch and exact-solver fallback).
+//              CUDA's pow() (exact-solver fallback) or from the fifth roots and powers
+//              of the TRRS branch.  Quotients by a divisor that other quotients share
+//              are rounded as IEEE division rounds them, from one reciprocal.
 //   MathF32 -- the mixed path's reconstruction, wave speeds and fluxes in FP32:
 //              the same algorithm with one reciprocal per density, approximate
 //              (single-instruction) division, reciprocal and square root
@@ -43,26 +45,51 @@ constexpr unsigned kStNegDensity = 0x01, kStNegPstar = 0x02, kStNan = 0x04, kStT
 struct MathF64 {
   using R = double;
 
-  // minmod_W, beta = 1 (src/hydro_utils.c:201)
+  // a / b from y = 1 / b rounded to nearest: the product and one fused correction,
+  // q' = q + (a - b q) y (P. Markstein, IBM J. Res. Dev. 34 (1990) 111).  The correction
+  // rounds to the IEEE quotient for a correctly rounded y; for a y one ulp off
+  // (div_yy) it may miss by an ulp where a/b lies within about 2^-105 of a
+  // rounding boundary.  3 FP64 instructions instead of a division's 8 to 9 and
+  // its range check, which made the divisions more than half of the FP64
+  // instructions of a face.  Where the quotient or the remainder leaves the
+  // normal range (b 0, infinite, below 1e-290; a infinite) the result may be
+  // infinite or a NaN instead of the quotient: the callers divide again when their
+  // result is not finite.
+  static __device__ __forceinline__ double div_y(double a, double b, double y) {
+    const double q = a * y;
+    return __fma_rn(__fma_rn(-b, q, a), y, q);
+  }
+  // a / RN(b b) from y = 1 / b: y y refined by one Newton step is the reciprocal
+  static __device__ __forceinline__ double div_yy(double a, double b, double y) {
+    const double bb = b * b, y0 = y * y;
+    return div_y(a, bb, __fma_rn(y0, __fma_rn(-bb, y0, 1.), y0));
+  }
+  // p / (gamma - 1) and friends: the divisor is a constant
+  static __device__ __forceinline__ double over_g1(double p) { return div_y(p, kGam - 1., 1. / (kGam - 1.)); }
+
+  // minmod_W, beta = 1 (src/hydro_utils.c:201): 0 if the signs differ, else the
+  // smaller magnitude.  One FP64 compare and selects on the sign bits instead of
+  // the reference's nested minima and maxima, each of which costs an FP64
+  // compare, two selects and a NaN check (15 limits a cell); equal for every pair
+  // of numbers but for the sign of a zero.
   static __device__ __forceinline__ double limit(double m, double p) {
-    if (p > 0) return fmax(fmax(0., fmin(m, p)), fmin(m, p));
-    return fmin(fmin(0., fmax(m, p)), fmax(m, p));
+    const double s = (fabs(m) < fabs(p)) ? m : p;
+    return ((__double2hiint(m) ^ __double2hiint(p)) < 0) ? 0. : s;
   }
 
   // MUSCL_BOUND2 slopes + matrix_jacobian predictor (src/hydro_utils.c:976-1189).
-  // q0: cell, qm/qp: neighbours per axis.  Out: D[3][5] slopes, Wt[5] predictor.
-  // azero: the cell's stored sound speed is 0 (an averaged split cell)
+  // q0: cell, qm/qp: neighbours per axis, fac = -dt/dx/2.  Out: D[3][5] slopes,
+  // Wt[5] predictor.  azero: the cell's stored sound speed is 0 (an averaged split cell)
   static __device__ __forceinline__ void muscl(const double q0[5], const double qm[3][5], const double qp[3][5],
-                                               double dt, double dx, double D[3][5], double Wt[5],
-                                               bool azero = false) {
+                                               double fac, double D[3][5], double Wt[5], bool azero = false) {
 #pragma unroll
     for (int dir = 0; dir < 3; dir++)
 #pragma unroll
       for (int k = 0; k < 5; k++) D[dir][k] = limit(q0[k] - qm[dir][k], qp[dir][k] - q0[k]);
     // stored sound speed of the cell, as U2W/scatter computes it (src/hydro_utils.c:64,3186)
-    const double a0 = azero ? 0. : sqrt(kGam * q0[4] / q0[0]);
-    const double daa = q0[0] * a0 * a0;
     const double id = 1. / q0[0];
+    const double a0 = azero ? 0. : sqrt(div_y(kGam * q0[4], q0[0], id));
+    const double daa = q0[0] * a0 * a0;
     double acc[5] = {0., 0., 0., 0., 0.};
 #pragma unroll
     for (int dir = 0; dir < 3; dir++) {
@@ -80,15 +107,18 @@ struct MathF64 {
       acc[1 + dir] += id * D[dir][4];
       acc[4] += s * D[dir][4];
     }
-    const double fac = -dt / dx * 0.5;
 #pragma unroll
     for (int i = 0; i < 5; i++) Wt[i] = acc[i] * fac;
   }
 
-  // E and a of a face state from its (d,u,v,w,p)
+  // 1/d and a of a face state from its (d,u,v,w,p): W = {d,u,v,w,p,1/d,a}
   static __device__ __forceinline__ void face_finish(double W[7]) {
-    W[6] = W[4] / (kGam - 1.) + 0.5 * W[0] * (W[1] * W[1] + W[2] * W[2] + W[3] * W[3]);
-    W[5] = sqrt(kGam * W[4] / W[0]);
+    W[5] = 1. / W[0];
+    W[6] = sqrt(div_y(kGam * W[4], W[0], W[5]));
+  }
+  // E of a face state (getE, src/hydro_utils.c:29)
+  static __device__ __forceinline__ double energy(const double W[7]) {
+    return over_g1(W[4]) + 0.5 * W[0] * (W[1] * W[1] + W[2] * W[2] + W[3] * W[3]);
   }
 
   struct S1 { double d, u, p, a; };
@@ -145,15 +175,44 @@ struct MathF64 {
     return p;
   }
 
+  // x^5 = h + l to twice the working precision
+  static __device__ __forceinline__ void pow5(double x, double &h, double &l) {
+    const double x2 = x * x, e2 = __fma_rn(x, x, -x2);
+    const double x4 = x2 * x2, e4 = __fma_rn(2. * x2, e2, __fma_rn(x2, x2, -x4));
+    h = x4 * x;
+    l = __fma_rn(e4, x, __fma_rn(x4, x, -h));
+  }
+  // pow(x, z) for z = the double nearest 1/5, x > 0, to within 0.51 ulp (so nearly always the
+  // bits of a correctly rounded pow): an FP32 estimate w of x^(-1/5) good to 2^-20, one
+  // step of the series of (1 - h)^(-1/5) = 1 + h/5 + 3 h^2/25 + ..., h = 1 - x w^5, which
+  // leaves an error of an ulp or two, y = x w^4, and a Newton correction from the residual
+  // x - y^5 at twice the precision, plus y (z - 1/5) ln x.  Some 30 FP64 instructions
+  // where pow() takes a hundred or more.
+  static __device__ __forceinline__ double root5(double x) {
+    const float xf = (float)x;
+    if (!(xf > 1e-37f && xf < 1e37f)) return pow(x, 0.2);  // outside the estimate's range
+    const float lg = __log2f(xf);
+    const double w0 = (double)exp2f(-0.2f * lg), v0 = w0 * w0;
+    const double h = __fma_rn(-x, v0 * v0 * w0, 1.);
+    const double w = __fma_rn(w0, h * __fma_rn(h, 3. / 25., 1. / 5.), w0);
+    const double w2 = w * w, w4 = w2 * w2, y = x * w4;
+    double y5, e5;
+    pow5(y, y5, e5);
+    constexpr double kZ = 1.1102230246251565e-17 * 0.6931471805599453;  // (z - 1/5) ln 2
+    return y + __fma_rn((x - y5) - e5, 0.2 * w4, y * ((double)lg * kZ));
+  }
+
   // Two-rarefaction star state of findPressure_Hybrid (src/hydro_utils.c:645-650),
-  // {p*, u*}.  Not inlined: its pow() expansions would otherwise be repeated in
-  // every copy of the Riemann solver and crowd the instruction cache.
+  // {p*, u*}, the exponents 1/5 and 5 (a negative ratio, a vacuum-generating pair, gives
+  // p* < 0 as pow() with an odd integer exponent does, and the exact solver replaces
+  // both).  Not inlined: it would crowd the instruction cache in every copy of the solver.
   static __device__ __noinline__ double2 trrs(double aL, double aR, double uL, double uR, double pL, double pR) {
-    const double z = (kGam - 1.) / (2. * kGam);
-    const double iz = (2. * kGam) / (kGam - 1.);
-    const double pstar = pow((aL + aR - (kGam - 1.) / 2. * (uR - uL)) / (aL / pow(pL, z) + aR / pow(pR, z)), iz);
-    const double ustar = uL - 2. * aL / (kGam - 1.) * (pow(pstar / pL, z) - 1.);
-    return make_double2(pstar, ustar);
+    static_assert((kGam - 1.) / (2. * kGam) == 0.2 && (2. * kGam) / (kGam - 1.) == 5., "fifth roots need gamma = 5/3");
+    const double r = (aL + aR - (kGam - 1.) / 2. * (uR - uL)) / (aL / root5(pL) + aR / root5(pR));
+    double h, l;
+    pow5(r, h, l);
+    const double pstar = h + l;
+    return make_double2(pstar, uL - over_g1(2. * aL) * (root5(pstar / pL) - 1.));
   }
 
   // findPressure_Hybrid + speedestimate*_HLLC (src/hydro_utils.c:625,1264)
@@ -161,13 +220,14 @@ struct MathF64 {
                                                 double &ustar, unsigned &st) {
     const double uLn = (n == 0) ? WL[1] : ((n == 1) ? WL[2] : WL[3]);
     const double uRn = (n == 0) ? WR[1] : ((n == 1) ? WR[2] : WR[3]);
-    S1 L{WL[0], uLn, WL[4], sqrt(kGam * WL[4] / WL[0])};
-    S1 R{WR[0], uRn, WR[4], sqrt(kGam * WR[4] / WR[0])};
+    S1 L{WL[0], uLn, WL[4], WL[6]};
+    S1 R{WR[0], uRn, WR[4], WR[6]};
     double dbar = 0.5 * (L.d + R.d), abar = 0.5 * (L.a + R.a);
     double ppvrs = 0.5 * ((L.p + R.p) + (L.u - R.u) * dbar * abar);
     double pmax = fmax(L.p, R.p), pmin = fmin(L.p, R.p);
     double pstar = ppvrs;
-    if (((pmax / pmin) < 2.) && ((pmin < pstar) && (pstar < pmax))) {
+    // pmax / pmin < 2: the rounded quotient is below 2 exactly where pmax < 2 pmin
+    if ((pmax < 2. * pmin) && ((pmin < pstar) && (pstar < pmax))) {
       ustar = 0.5 * ((L.u + R.u) + (L.p - R.p) / (dbar * abar));
     } else if (pstar < pmin) {
       const double2 r = trrs(L.a, R.a, L.u, R.u, L.p, R.p);
@@ -213,28 +273,43 @@ struct MathF64 {
     face_finish(W);
   }
 
-  // State rotated to the face frame: r = {d, u_n, u_t1, u_t2, p, E, |m|^2},
+  // State rotated to the face frame: r = {d, u_n, u_t1, u_t2, p, E, |m|^2, 1/d},
   // t1 < t2 the transverse axes in x,y,z order, |m|^2 summed in x,y,z order.
-  static __device__ __forceinline__ void rotate(const double W[7], int n, double r[7]) {
+  static __device__ __forceinline__ void rotate(const double W[7], int n, double r[8]) {
     r[0] = W[0];
     r[1] = (n == 0) ? W[1] : ((n == 1) ? W[2] : W[3]);
     r[2] = (n == 0) ? W[2] : W[1];
     r[3] = (n == 2) ? W[2] : W[3];
     r[4] = W[4];
-    r[5] = W[6];
+    r[5] = energy(W);
     const double m0 = W[0] * W[1], m1 = W[0] * W[2], m2 = W[0] * W[3];
     r[6] = m0 * m0 + m1 * m1 + m2 * m2;
+    r[7] = W[5];
   }
 
-  // getflux_{X,Y,Z} of W2U(W) (src/hydro_utils.c:66,916-968) in the face frame
-  static __device__ __forceinline__ void euler_rot(const double r[7], double f[5]) {
-    const double d = r[0], E = r[5];
+  // getflux_{X,Y,Z} of W2U(W) (src/hydro_utils.c:66,916-968) in the face frame: the
+  // reference's quotients by d and d^2 from 1/d, or (IEEE) by division
+  template <bool IEEE>
+  static __device__ __forceinline__ void euler_quot(const double r[8], double f[5]) {
+    const double d = r[0], E = r[5], y = r[7];
     const double mn = d * r[1], mt1 = d * r[2], mt2 = d * r[3];
+    auto over_d = [&](double a) { return IEEE ? a / d : div_y(a, d, y); };
     f[0] = mn;
-    f[1] = 0.5 * (3. - kGam) * mn * mn / d + (kGam - 1.) * E - 0.5 * (kGam - 1.) * (mt1 * mt1 + mt2 * mt2) / d;
-    f[2] = mn * mt1 / d;
-    f[3] = mn * mt2 / d;
-    f[4] = kGam * mn / d * E - 0.5 * (kGam - 1.) * mn / (d * d) * r[6];
+    f[1] = over_d(0.5 * (3. - kGam) * mn * mn) + (kGam - 1.) * E - over_d(0.5 * (kGam - 1.) * (mt1 * mt1 + mt2 * mt2));
+    f[2] = over_d(mn * mt1);
+    f[3] = over_d(mn * mt2);
+    const double c = 0.5 * (kGam - 1.) * mn;
+    f[4] = over_d(kGam * mn) * E - (IEEE ? c / (d * d) : div_yy(c, d, y)) * r[6];
+  }
+  static __device__ __noinline__ void euler_ieee(const double r[8], double f[5]) { euler_quot<true>(r, f); }
+  static __device__ __forceinline__ void euler_rot(const double r[8], double f[5]) {
+    euler_quot<false>(r, f);
+    if (!isfinite(f[4])) {  // a quotient may have left div_y's range (every term of f enters f[4])
+      double t[8], u[5];
+      for (int i = 0; i < 8; i++) t[i] = r[i];
+      euler_ieee(t, u);
+      for (int i = 0; i < 5; i++) f[i] = u[i];
+    }
   }
 
   // HLLC flux across a face normal to axis n (src/hydro_utils.c:2055-2138),
@@ -250,35 +325,36 @@ struct MathF64 {
                                               double *fx = nullptr) {
     double SL, SR, ustar;
     speeds(WL, WR, n, SL, SR, ustar, st);
-    double rL[7], rR[7], G[5] = {0., 0., 0., 0., 0.};
-    rotate(WL, n, rL);
-    rotate(WR, n, rR);
+    double G[5] = {0., 0., 0., 0., 0.};
     if (du != nullptr) du[0] = du[1] = 0.;
     if (fx != nullptr)
       for (int t = 0; t < NT; t++) fx[t] = 0.;
-    if (SL >= 0. || SR <= 0.) {
-      const double *r = (SL >= 0.) ? rL : rR;
+    // the upwind side's flux, plus the star correction inside the fan; no flux when
+    // neither side's condition holds (a NaN speed)
+    const bool upwind = SL >= 0. || SR <= 0.;
+    const bool left = upwind ? (SL >= 0.) : ((SL < 0.) && (ustar >= 0.));
+    const bool right = upwind || ((ustar <= 0.) && (SR > 0.));
+    if (left || right) {
+      double W[7], r[8];
+#pragma unroll
+      for (int i = 0; i < 6; i++) W[i] = left ? WL[i] : WR[i];
+      rotate(W, n, r);
       euler_rot(r, G);
-      if (du != nullptr) {  // Us = W2U of the upwind face state
-        const double mn = r[0] * r[1];
-        du[0] = mn / r[0];
-        du[1] = (r[5] - 0.5 * r[6] / r[0]);
-      }
-      if (fx != nullptr)  // tracers: face values from the centre fractions, flux du dT / d
-        for (int t = 0; t < NT; t++) {
-          const double dT = (r[0] * Tracers<NT>::frac(t)) * xs[2 * t + ((SL >= 0.) ? 0 : 1)];
-          fx[t] = (r[0] * r[1]) * dT / r[0];
+      const double d = r[0], un = r[1], E = r[5], y = r[7];
+      if (upwind) {
+        if (du != nullptr) {  // Us = W2U of the upwind face state
+          du[0] = div_y(d * un, d, y);
+          du[1] = (E - div_y(0.5 * r[6], d, y));
         }
-    } else {
-      const bool left = (SL < 0.) && (ustar >= 0.);
-      const bool right = (ustar <= 0.) && (SR > 0.);
-      if (left || right) {
-        const double *r = left ? rL : rR;
+        if (fx != nullptr)  // tracers: face values from the centre fractions, flux du dT / d
+          for (int t = 0; t < NT; t++) {
+            const double dT = (d * Tracers<NT>::frac(t)) * xs[2 * t + (left ? 0 : 1)];
+            fx[t] = div_y((d * un) * dT, d, y);
+          }
+      } else {
         const double S = left ? SL : SR;
-        euler_rot(r, G);
-        const double d = r[0], un = r[1], E = r[5];
         const double fact = d * (S - un) / (S - ustar);
-        const double Es = (E / d + (ustar - un) * (ustar + r[4] / (d * (S - un))));
+        const double Es = (div_y(E, d, y) + (ustar - un) * (ustar + r[4] / (d * (S - un))));
         G[0] += (fact * 1. - d) * S;
         G[1] += (fact * ustar - d * un) * S;
         G[2] += (fact * r[2] - d * r[2]) * S;
@@ -287,7 +363,7 @@ struct MathF64 {
         if (fx != nullptr)  // tracer fluxes with the star correction (src/hydro_utils.c:1534-1539)
           for (int t = 0; t < NT; t++) {
             const double dT = (d * Tracers<NT>::frac(t)) * xs[2 * t + (left ? 0 : 1)];
-            fx[t] = (d * un) * dT / d + (fact * dT / d - dT) * S;
+            fx[t] = div_y((d * un) * dT, d, y) + (div_y(fact * dT, d, y) - dT) * S;
           }
         if (du != nullptr) {  // the star state: momenta in x,y,z order for the sum of squares
           const double ds = fact * 1., mn = fact * ustar, m1 = fact * r[2], m2 = fact * r[3];

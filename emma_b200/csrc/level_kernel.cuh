@@ -556,6 +556,8 @@ __device__ __forceinline__ void level_tile(const BatchArgs &Bt, const LevelArgs 
   // contributes).  One call site each for the reconstruction and the face
   // state, so that a face on a brick boundary, solved by both bricks, rounds
   // the same in both.
+  const double dtsurdx = A.dt / A.dx;
+  const R hfac = F64 ? (R)(-dtsurdx * 0.5) : (R)(dtsurdx * 0.5);  // the predictor's half step (FP32: its sign in muscl)
 #pragma unroll 1
   for (int w = tid; w < kThreads + NRING; w += kThreads) {
     int b = tb, k = 0, r = 0;
@@ -591,8 +593,7 @@ __device__ __forceinline__ void level_tile(const BatchArgs &Bt, const LevelArgs 
     q_at(b - G::XS, qm[2]);
     q_at(b + G::XS, qp[2]);
     const bool azero = DUAL && (sSt[b] & kFAzero);
-    if constexpr (F64) M::muscl(q0, qm, qp, A.dt, A.dx, D, Wt, azero);
-    else M::muscl(q0, qm, qp, (R)(A.dt / A.dx * 0.5), D, Wt, azero);
+    M::muscl(q0, qm, qp, hfac, D, Wt, azero);
     // X = W0 + Wt (FP32 path) or Wt (FP64 path, which adds W0 in the reference's order)
 #pragma unroll
     for (int v = 0; v < 5; v++) X[v] = F64 ? Wt[v] : q0[v] + Wt[v];
@@ -781,10 +782,7 @@ __device__ __forceinline__ void level_tile(const BatchArgs &Bt, const LevelArgs 
   auto face_sums = [&](int k0, int k1) {
     const uint8_t f = sSt[tb];
     if (!(f & kFTile) || (f & kFSplit)) return;
-    const double dtsurdx = A.dt / A.dx;
-    R q4;
-    q4 = sMp[tid];
-    const double eold = (double)q4 / (kGam - 1.);
+    const double eold = MathF64::over_g1((double)sMp[tid]);
 #pragma unroll
     for (int k = k0; k < k1; k++) {
       const int d = k >> 1, up = k & 1;
@@ -990,7 +988,6 @@ __device__ __forceinline__ void level_tile(const BatchArgs &Bt, const LevelArgs 
 #pragma unroll
       for (int v = 0; v < 5; v++) Wout[v] = acc[v];
     } else {
-      const double dtsurdx = A.dt / A.dx;
       // face e of this cell: -x,+x,-y,+y,-z,+z
       const int eb = tn * G::kFaces;
       const int ex = eb + G::face_index(0, tx, ty, tz), ey = eb + G::face_index(1, tx, ty, tz),
@@ -1028,15 +1025,15 @@ __device__ __forceinline__ void level_tile(const BatchArgs &Bt, const LevelArgs 
         Udv = bd * A.B[2 * N8 + gi];
         Udw = bd * A.B[3 * N8 + gi];
         UE = A.B[5 * N8 + gi];
-        if constexpr (DUAL) Ue = A.B[4 * N8 + gi] / (kGam - 1.);
+        if constexpr (DUAL) Ue = MathF64::over_g1(A.B[4 * N8 + gi]);
       } else {  // resident: W2U(field) + corrections received from the finer level
         Ud = q[0];
         Udu = q[0] * q[1];
         Udv = q[0] * q[2];
         Udw = q[0] * q[3];
-        UE = q[4] / (kGam - 1.) + 0.5 * q[0] * (q[1] * q[1] + q[2] * q[2] + q[3] * q[3]);
+        UE = MathF64::over_g1(q[4]) + 0.5 * q[0] * (q[1] * q[1] + q[2] * q[2] + q[3] * q[3]);
         if constexpr (DUAL) {
-          Ue = q[4] / (kGam - 1.);
+          Ue = MathF64::over_g1(q[4]);
           if (A.C != nullptr) Ue += take_c(5);
         }
       }
@@ -1048,7 +1045,7 @@ __device__ __forceinline__ void level_tile(const BatchArgs &Bt, const LevelArgs 
         dUe = aUe;
         divu = aDivu;
       } else if constexpr (DUAL) {
-        const double eold = q[4] / (kGam - 1.);
+        const double eold = MathF64::over_g1(q[4]);
         double one = 1.;
 #pragma unroll
         for (int k = 0; k < 6; k++) {
@@ -1122,11 +1119,20 @@ __device__ __forceinline__ void level_tile(const BatchArgs &Bt, const LevelArgs 
       // U2W (src/hydro_utils.c:35-64), pressure floor, E - Ekin recovery
       const double dl = (Ud == 0. ? 10. : Ud);
       Wout[0] = Ud;
+      double ydl = 0.;  // 1 / dl
       if constexpr (F64) {
-        Wout[1] = Udu / dl;
-        Wout[2] = Udv / dl;
-        Wout[3] = Udw / dl;
-        Wout[4] = (kGam - 1.) * (UE - ((Udu) * (Udu) + (Udv) * (Udv) + (Udw) * (Udw)) / (dl) * 0.5);
+        const double mm = (Udu) * (Udu) + (Udv) * (Udv) + (Udw) * (Udw);
+        ydl = 1. / dl;
+        Wout[1] = MathF64::div_y(Udu, dl, ydl);
+        Wout[2] = MathF64::div_y(Udv, dl, ydl);
+        Wout[3] = MathF64::div_y(Udw, dl, ydl);
+        Wout[4] = (kGam - 1.) * (UE - MathF64::div_y(mm, dl, ydl) * 0.5);
+        if (!isfinite(Wout[4])) {  // out of div_y's range: by division
+          Wout[1] = Udu / dl;
+          Wout[2] = Udv / dl;
+          Wout[3] = Udw / dl;
+          Wout[4] = (kGam - 1.) * (UE - mm / dl * 0.5);
+        }
       } else {
         const double inv = 1. / dl;  // mixed path: one FP64 division per cell
         Wout[1] = Udu * inv;
@@ -1141,7 +1147,7 @@ __device__ __forceinline__ void level_tile(const BatchArgs &Bt, const LevelArgs 
         double eint = Ue + dUe;
         eint = eint + (-divu * dtsurdx);
         if ((UE - ekin) > 0.5 * (divu * divu)) eint = UE - ekin;
-        eint = fmax(eint * (kGam - 1.), kPmin) / (kGam - 1.);
+        eint = MathF64::over_g1(fmax(eint * (kGam - 1.), kPmin));
         Wout[4] = eint * (kGam - 1.);
       }
       Wout[4] = fmax(Wout[4], kPmin);
