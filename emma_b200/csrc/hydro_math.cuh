@@ -59,6 +59,28 @@ struct MathF64 {
     const double q = a * y;
     return __fma_rn(__fma_rn(-b, q, a), y, q);
   }
+  // 1 / b and sqrt(x) rounded to nearest for arguments and results in the normal range
+  // (a NaN where they are not, an ulp off where the exact value lies within about
+  // 2^-100 of a rounding boundary): a 20-bit seed (PTX rcp.approx / rsqrt.approx),
+  // one step of the binomial series, and Markstein's correction from the exact
+  // residual.  As many FP64 instructions as the IEEE operators, without their range
+  // checks and branches, three a division, which are every fourth instruction of a face.
+  static __device__ __forceinline__ double rcp(double b) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    const double e = __fma_rn(-b, y, 1.);
+    y = __fma_rn(y, __fma_rn(e, e, e), y);
+    return __fma_rn(y, __fma_rn(-b, y, 1.), y);
+  }
+  static __device__ __forceinline__ double root2(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double t = x * y, e = __fma_rn(-t, y, 1.);
+    const double g = __fma_rn(t, e * __fma_rn(e, 0.375, 0.5), t);
+    return __fma_rn(__fma_rn(-g, g, x), 0.5 * y, g);
+  }
+  static __device__ __forceinline__ double quot(double a, double b) { return div_y(a, b, rcp(b)); }
+
   // a / RN(b b) from y = 1 / b: y y refined by one Newton step is the reciprocal
   static __device__ __forceinline__ double div_yy(double a, double b, double y) {
     const double bb = b * b, y0 = y * y;
@@ -87,8 +109,8 @@ struct MathF64 {
 #pragma unroll
       for (int k = 0; k < 5; k++) D[dir][k] = limit(q0[k] - qm[dir][k], qp[dir][k] - q0[k]);
     // stored sound speed of the cell, as U2W/scatter computes it (src/hydro_utils.c:64,3186)
-    const double id = 1. / q0[0];
-    const double a0 = azero ? 0. : sqrt(div_y(kGam * q0[4], q0[0], id));
+    const double id = rcp(q0[0]);
+    const double a0 = azero ? 0. : root2(div_y(kGam * q0[4], q0[0], id));
     const double daa = q0[0] * a0 * a0;
     double acc[5] = {0., 0., 0., 0., 0.};
 #pragma unroll
@@ -113,8 +135,8 @@ struct MathF64 {
 
   // 1/d and a of a face state from its (d,u,v,w,p): W = {d,u,v,w,p,1/d,a}
   static __device__ __forceinline__ void face_finish(double W[7]) {
-    W[5] = 1. / W[0];
-    W[6] = sqrt(div_y(kGam * W[4], W[0], W[5]));
+    W[5] = rcp(W[0]);
+    W[6] = root2(div_y(kGam * W[4], W[0], W[5]));
   }
   // E of a face state (getE, src/hydro_utils.c:29)
   static __device__ __forceinline__ double energy(const double W[7]) {
@@ -208,11 +230,11 @@ struct MathF64 {
   // both).  Not inlined: it would crowd the instruction cache in every copy of the solver.
   static __device__ __noinline__ double2 trrs(double aL, double aR, double uL, double uR, double pL, double pR) {
     static_assert((kGam - 1.) / (2. * kGam) == 0.2 && (2. * kGam) / (kGam - 1.) == 5., "fifth roots need gamma = 5/3");
-    const double r = (aL + aR - (kGam - 1.) / 2. * (uR - uL)) / (aL / root5(pL) + aR / root5(pR));
+    const double r = quot(aL + aR - (kGam - 1.) / 2. * (uR - uL), quot(aL, root5(pL)) + quot(aR, root5(pR)));
     double h, l;
     pow5(r, h, l);
     const double pstar = h + l;
-    return make_double2(pstar, uL - over_g1(2. * aL) * (root5(pstar / pL) - 1.));
+    return make_double2(pstar, uL - over_g1(2. * aL) * (root5(quot(pstar, pL)) - 1.));
   }
 
   // findPressure_Hybrid + speedestimate*_HLLC (src/hydro_utils.c:625,1264)
@@ -228,23 +250,29 @@ struct MathF64 {
     double pstar = ppvrs;
     // pmax / pmin < 2: the rounded quotient is below 2 exactly where pmax < 2 pmin
     if ((pmax < 2. * pmin) && ((pmin < pstar) && (pstar < pmax))) {
-      ustar = 0.5 * ((L.u + R.u) + (L.p - R.p) / (dbar * abar));
+      ustar = 0.5 * ((L.u + R.u) + quot(L.p - R.p, dbar * abar));
     } else if (pstar < pmin) {
       const double2 r = trrs(L.a, R.a, L.u, R.u, L.p, R.p);
       pstar = r.x;
       ustar = r.y;
     } else {
       double p0 = fmax(0., ppvrs);
-      double AL = 2. / ((kGam + 1.) * L.d), AR = 2. / ((kGam + 1.) * R.d);
+      // A = 2 / ((gamma + 1) d): the reciprocal of the rounded (gamma + 1) d from 1 / d
+      auto two_over = [](double d, double y) {
+        const double b = (kGam + 1.) * d, y0 = y * (1. / (kGam + 1.));
+        return 2. * __fma_rn(y0, __fma_rn(-b, y0, 1.), y0);
+      };
+      double AL = two_over(L.d, WL[5]), AR = two_over(R.d, WR[5]);
       double BL = (kGam - 1.) / (kGam + 1.) * L.p, BR = (kGam - 1.) / (kGam + 1.) * R.p;
-      double GL = sqrt(AL / (p0 + BL)), GR = sqrt(AR / (p0 + BR));
-      pstar = (GL * L.p + GR * R.p - (R.u - L.u)) / (GL + GR);
+      double GL = root2(quot(AL, p0 + BL)), GR = root2(quot(AR, p0 + BR));
+      pstar = quot(GL * L.p + GR * R.p - (R.u - L.u), GL + GR);
       ustar = 0.5 * ((L.u + R.u) + (pstar - R.p) * GR - (pstar - L.p) * GL);
     }
     if (pstar < 0) pstar = pstar_exact(L, R, &ustar, st);
     if (pstar < 0) st |= kStNegPstar;
-    double qL = (pstar <= WL[4] ? 1. : sqrt(1. + (kGam + 1.) / (2. * kGam) * ((pstar) / WL[4] - 1.)));
-    double qR = (pstar <= WR[4] ? 1. : sqrt(1. + (kGam + 1.) / (2. * kGam) * ((pstar) / WR[4] - 1.)));
+    double qL = 1., qR = 1.;
+    if (!(pstar <= WL[4])) qL = root2(1. + (kGam + 1.) / (2. * kGam) * (quot(pstar, WL[4]) - 1.));
+    if (!(pstar <= WR[4])) qR = root2(1. + (kGam + 1.) / (2. * kGam) * (quot(pstar, WR[4]) - 1.));
     SL = L.u - L.a * qL;
     SR = R.u + R.a * qR;
     if (SL > SR) {
@@ -257,7 +285,8 @@ struct MathF64 {
   // Face state toward face k from the slope along k's axis only (the other
   // axes enter the reference's sum with coefficient 0).
   // g (optional): the gravity kick -f dt/2 of the face velocities, added after
-  // the pressure floor and before E and a (src/hydro_utils.c:1219-1226)
+  // the pressure floor and before E and a (src/hydro_utils.c:1219-1226).  W[5], W[6]
+  // are left to face_finish.
   static __device__ __forceinline__ void face_ax(const double q0[5], const double Dax[5], const double Wt[5], int k,
                                                  double W[7], unsigned &st, const double *g = nullptr) {
     const double f = (k & 1) ? 0.5 : -0.5;
@@ -270,7 +299,6 @@ struct MathF64 {
       W[2] += g[1];
       W[3] += g[2];
     }
-    face_finish(W);
   }
 
   // State rotated to the face frame: r = {d, u_n, u_t1, u_t2, p, E, |m|^2, 1/d},
@@ -353,8 +381,8 @@ struct MathF64 {
           }
       } else {
         const double S = left ? SL : SR;
-        const double fact = d * (S - un) / (S - ustar);
-        const double Es = (div_y(E, d, y) + (ustar - un) * (ustar + r[4] / (d * (S - un))));
+        const double fact = quot(d * (S - un), S - ustar);
+        const double Es = (div_y(E, d, y) + (ustar - un) * (ustar + quot(r[4], d * (S - un))));
         G[0] += (fact * 1. - d) * S;
         G[1] += (fact * ustar - d * un) * S;
         G[2] += (fact * r[2] - d * r[2]) * S;

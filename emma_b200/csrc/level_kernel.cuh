@@ -671,8 +671,7 @@ __device__ __forceinline__ void level_tile(const BatchArgs &Bt, const LevelArgs 
   auto ring_face = [&](int r, R W[7]) {
     V::ld(sHS, r, NRING, W[0], W[1], W[2], W[3]);
     if constexpr (F64) {
-      W[4] = sHS[4 * NRING + r];
-      M::face_finish(W);
+      W[4] = sHS[4 * NRING + r];  // 1/d and a: solve_face, ring and brick lanes together
     } else {
       R pad;
       V::ld(sHS, NRING + r, NRING, W[4], W[5], W[6], pad);
@@ -691,6 +690,10 @@ __device__ __forceinline__ void level_tile(const BatchArgs &Bt, const LevelArgs 
       else brick_face(tL, bL, 2 * d + 1, WL);
       if (jR >= 0) ring_face(jR, WR);
       else brick_face(tR, bR, 2 * d, WR);
+      if constexpr (F64) {
+        M::face_finish(WL);
+        M::face_finish(WR);
+      }
       if constexpr (TRACER) {
         R xs[2 * NTR];
 #pragma unroll
@@ -1122,7 +1125,7 @@ __device__ __forceinline__ void level_tile(const BatchArgs &Bt, const LevelArgs 
       double ydl = 0.;  // 1 / dl
       if constexpr (F64) {
         const double mm = (Udu) * (Udu) + (Udv) * (Udv) + (Udw) * (Udw);
-        ydl = 1. / dl;
+        ydl = MathF64::rcp(dl);
         Wout[1] = MathF64::div_y(Udu, dl, ydl);
         Wout[2] = MathF64::div_y(Udv, dl, ydl);
         Wout[3] = MathF64::div_y(Udw, dl, ydl);
