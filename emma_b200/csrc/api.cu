@@ -34,7 +34,8 @@ cudaError_t launch_level_fp64(const BatchArgs &a, unsigned shapes, int nsm, int 
                               int *occupancy);
 cudaError_t launch_level_f32(const BatchArgs &a, unsigned shapes, int nsm, int ctas_per_sm, cudaStream_t s,
                              int *occupancy);
-cudaError_t launch_column_f32(const ColumnArgs &a, cudaStream_t s);
+cudaError_t launch_column_f32(const ColumnArgs &a, unsigned variant, cudaStream_t s);
+cudaError_t launch_column_fp64(const ColumnArgs &a, unsigned variant, cudaStream_t s);
 cudaError_t launch_step_f32(const StepArgs &a, unsigned variant, int groups, int nsm, cudaStream_t s, int *grid,
                             int *threads);
 cudaError_t launch_step_fp64(const StepArgs &a, unsigned variant, int groups, int nsm, cudaStream_t s, int *grid,
@@ -77,21 +78,24 @@ struct DevLevel {
   double *F = nullptr;     // gravity build: acceleration planes fx,fy,fz of the level's cells
   double *Fv = nullptr;    // gravity build: interpolated accelerations of the listed coarser cells
   uint8_t *az = nullptr;   // dual energy: per cell, a split cell whose stored sound speed is 0
-  // column kernel (column_kernel.cuh): a complete periodic level without split cells of a
-  // resident plain-variant tree has the oct index of every oct position; col_nz is the
-  // planes per work item the autotuner chose (0: the brick kernel was faster)
+  // column kernel (column_kernel.cuh): a complete level without split cells, periodic or
+  // transmissive in x, of a resident tree has the oct index of every oct position; the
+  // autotuner's choices are kept per precision (EMMA_PREC_*): nz the planes per work
+  // item (0: the brick kernel was faster)
   int *octidx = nullptr;
   int col_n = 0;  // octs per side, 0 when the level is not eligible
   // device-side refinement (refine_impl.cuh, resident levels): the oct of this level
   // across each face of every oct (-1: none), and the refinement mark of every cell
   int *nb6 = nullptr;
   int *marks = nullptr;
-  int col_nz = 0;
-  double col_sweep_ms[6] = {};  // planes per item 2, 4, 8, 16, 32, 64 (0 = not tried)
-  int col_xs = 0;               // the autotuner's x sweep: 1 warp shuffles, 0 shared memory
-  double col_xs_ms[2] = {};     // its times of the two at col_nz (0 = not timed)
-  int col_bal = 0;              // the autotuner's work split: 1 balanced runs, 0 items
-  double col_bal_ms[2] = {};    // its times of the two (0 = not timed)
+  struct Column {
+    int nz = 0;
+    double sweep_ms[6] = {};  // planes per item 2, 4, 8, 16, 32, 64 (0 = not tried)
+    int xs = 0;               // x sweep: 1 warp shuffles, 0 shared memory
+    double xs_ms[2] = {};     // the times of the two at nz (0 = not timed)
+    int bal = 0;              // work split: 1 balanced runs, 0 items
+    double bal_ms[2] = {};    // the times of the two (0 = not timed)
+  } col[2];
   long long nv = 0;
   int shape = 0;        // brick shape of the plan (kShapes)
   int ctas = 0;         // CTAs per SM of its launches (0: the occupancy limit)
@@ -431,7 +435,7 @@ bool upload_vec(T **dst, const std::vector<T> &v) {
 
 // Allocate device arrays of the mirrored levels, copy topology + plans, and
 // initialise the device level slots.
-int column_default_nz(const DevLevel &d);
+int column_default_nz(const DevLevel &d, int prec);
 
 bool alloc_tree(const HostTree &H, Tree &t, bool with_base) {
   t.lev.assign(H.lev.size(), DevLevel());
@@ -533,10 +537,13 @@ bool alloc_tree(const HostTree &H, Tree &t, bool with_base) {
         for (int c = 0; c < 8; c++) m[8 * (size_t)i + c] = (int)h.octs[i]->cell[c].marked;
       if (!upload_vec(&d.marks, m)) return false;
     }
-    // the column kernel: a complete periodic level without split cells of a resident
-    // plain-variant tree (its oct at every position, so no tile plan is read)
+    // the column kernel: a complete level without split cells of a resident tree (its
+    // oct at every position, so no tile plan is read), periodic or transmissive in x (the
+    // ghosts across an x face are copies of the boundary cell; those across +y are not);
+    // not the combinations of variants it is not built for
     const long long nside = 1LL << (L - 1);
-    if (!with_base && !has_split && !H.trans && !H.grav && !g.opt.dual_energy && !kDropinTracer && L >= 4 &&
+    if (!with_base && !has_split && (H.trans & ~(EMMA_TRANS_XM | EMMA_TRANS_XP)) == 0 &&
+        !(H.grav && g.opt.dual_energy) && kDropinTracer <= 1 && L >= 4 &&
         h.noct == h.nown && (long long)h.noct == nside * nside * nside && (2 * nside) % kColumnWidth == 0) {
       std::vector<int> idx((size_t)h.noct, -1);
       bool full = true;
@@ -548,7 +555,7 @@ bool alloc_tree(const HostTree &H, Tree &t, bool with_base) {
       if (full) {
         if (!upload_vec(&d.octidx, idx)) return false;
         d.col_n = (int)nside;
-        d.col_nz = column_default_nz(d);
+        for (int p = 0; p < 2; p++) d.col[p].nz = column_default_nz(d, p);
       }
     }
     k_set_args<<<1, 1, 0, g.stream>>>(t.d_lv, L, a);
@@ -713,47 +720,60 @@ bool column_nz_ok(const DevLevel &d, int nz) {
   return d.col_n > 0 && nz >= 2 && nz % 2 == 0 && nz <= nc && nc % nz == 0;
 }
 
-long long column_items(const DevLevel &d, int nz) {
-  const long long ncol = 2LL * d.col_n / kColumnWidth;
-  return ncol * ncol * (2LL * d.col_n / nz);
+// columns of a level, and its work items of nz planes
+long long column_count(const DevLevel &d, int prec) {
+  const long long nc = 2LL * d.col_n;
+  return (nc / kColumnWidth) * (nc / column_height(prec == EMMA_PREC_FP64));
 }
+long long column_items(const DevLevel &d, int prec, int nz) { return column_count(d, prec) * (2LL * d.col_n / nz); }
 
 // the largest candidate that still gives every SM four work items (two CTAs per SM,
 // two waves), else the smallest valid one
-int column_default_nz(const DevLevel &d) {
+int column_default_nz(const DevLevel &d, int prec) {
   int best = 0;
   for (int nz : kColNz) {
     if (!column_nz_ok(d, nz)) continue;
-    if (best == 0 || column_items(d, nz) >= 4LL * g.nsm) best = nz;
+    if (best == 0 || column_items(d, prec, nz) >= 4LL * g.nsm) best = nz;
   }
   return best;
 }
 
+// the kernel variant of resident launches (launch flags; 0: plain)
+unsigned column_variant() {
+  return (g.res.host.grav ? kLaunchGrav : 0u) | (g.opt.dual_energy ? kLaunchDual : 0u) | kLaunchTracers;
+}
+
 // planes per item of a launch of resident level L on the column kernel; 0: the
-// brick kernel (FP64 path, ineligible level, option column < 0, or the
-// autotuner found the brick kernel faster)
+// brick kernel (ineligible level, option column < 0, a brick shape forced where
+// the option has always meant the brick kernel -- any but the plain mixed
+// variant on a periodic level --, or the autotuner found the brick kernel faster)
 int column_nz(int L) {
   if (L < 0 || !g.res.valid || L < g.res.lcoarse || L > g.res.lmax) return 0;
   const DevLevel &d = g.res.lev[L];
-  if (d.col_n == 0 || g.opt.precision != EMMA_PREC_MIXED || g.opt.column < 0) return 0;
+  if (d.col_n == 0 || g.opt.column < 0) return 0;
+  const bool mixed_plain = g.opt.precision == EMMA_PREC_MIXED && column_variant() == 0u && g.res.host.trans == 0;
+  if (!mixed_plain && g.opt.tile_octs != 0) return 0;
   if (g.opt.column > 0) return column_nz_ok(d, g.opt.column) ? g.opt.column : 0;
-  return d.col_nz;
+  return d.col[g.opt.precision == EMMA_PREC_MIXED].nz;
 }
 
-// x sweep of the column-kernel launches of resident level L (ColumnArgs::xshfl)
+// x sweep of the column-kernel launches of resident level L (ColumnArgs::xshfl): the
+// warp shuffles are the plain mixed variant's
 int column_xs(int L) {
+  if (g.opt.precision != EMMA_PREC_MIXED || column_variant() != 0u) return 0;
   if (g.opt.column_xshfl != 0) return g.opt.column_xshfl > 0 ? 1 : 0;
-  return g.opt.column > 0 ? 0 : g.res.lev[L].col_xs;
+  return g.opt.column > 0 ? 0 : g.res.lev[L].col[1].xs;
 }
 
 // work split of the column-kernel launches of resident level L (ColumnArgs::balanced)
 int column_bal(int L) {
   if (g.opt.column_balanced != 0) return g.opt.column_balanced > 0 ? 1 : 0;
-  return g.opt.column > 0 ? 0 : g.res.lev[L].col_bal;
+  return g.opt.column > 0 ? 0 : g.res.lev[L].col[g.opt.precision == EMMA_PREC_MIXED].bal;
 }
 
 cudaError_t launch_column(int L, int nz, const int *gate, bool fuse_cfl, int xs = -1, int bal = -1) {
   const DevLevel &d = g.res.lev[L];
+  const bool fp64 = g.opt.precision != EMMA_PREC_MIXED;
   ColumnArgs c;
   c.lv = g.res.d_lv + L;
   c.L = L;
@@ -761,18 +781,20 @@ cudaError_t launch_column(int L, int nz, const int *gate, bool fuse_cfl, int xs 
   c.n = d.col_n;
   c.nz = nz;
   c.ncol = 2 * d.col_n / kColumnWidth;
+  c.ncoly = 2 * d.col_n / column_height(fp64);
   c.balanced = bal >= 0 ? bal : column_bal(L);
-  if (c.balanced) {  // the kernel's two CTAs per SM, runs of at least 16 column-planes
-    const long long ncol = 2LL * d.col_n / kColumnWidth, planes = ncol * ncol * 2LL * d.col_n;
-    c.nitems = (int)std::max(1LL, std::min(2LL * g.nsm, planes / 16));
+  if (c.balanced) {  // the kernel's CTAs per SM, runs of at least 16 column-planes
+    const long long planes = column_count(d, g.opt.precision) * 2LL * d.col_n;
+    c.nitems = (int)std::max(1LL, std::min((long long)column_ctas(fp64) * g.nsm, planes / 16));
   } else {
-    c.nitems = (int)column_items(d, nz);
+    c.nitems = (int)column_items(d, g.opt.precision, nz);
   }
   c.gate = gate;
   c.status = g.d_status;
   c.smax = fuse_cfl ? g.d_S->smax_next : nullptr;
   c.xshfl = xs >= 0 ? xs : column_xs(L);
-  return launch_column_f32(c, g.stream);
+  c.trans = ((g.res.host.trans & EMMA_TRANS_XM) ? 1 : 0) | ((g.res.host.trans & EMMA_TRANS_XP) ? 2 : 0);
+  return fp64 ? launch_column_fp64(c, column_variant(), g.stream) : launch_column_f32(c, column_variant(), g.stream);
 }
 
 // fuse_cfl: the launch also accumulates each level's max signal speed of the
@@ -806,8 +828,7 @@ bool launch_batch(LevelArgs *d_lv, const int *work, int nwork, const int *gate, 
   if (grav || (d_lv == g.res.d_lv && g.res.host.grav)) shapes |= kLaunchGrav;
   if (g.opt.dual_energy) shapes |= kLaunchDual;
   shapes |= kLaunchTracers;
-  const int cnz = (d_lv == g.res.d_lv && !(shapes & (kLaunchGrav | kLaunchDual | kLaunchTracer | kLaunchHelium)))
-                      ? column_nz(col_level) : 0;
+  const int cnz = (d_lv == g.res.d_lv) ? column_nz(col_level) : 0;
   cudaError_t e = (cnz > 0) ? launch_column(col_level, cnz, gate, fuse_cfl)
                   : (g.opt.precision == EMMA_PREC_MIXED)
                       ? launch_level_f32(a, shapes, g.nsm, ctas, g.stream, nullptr)
@@ -1342,66 +1363,55 @@ bool autotune_tree(Tree &t, int shape_req) {
          ck(cudaStreamSynchronize(g.stream), "tune");
     d.ctas = best_ctas;
     d.tuned = ok;
-    // the column kernel against the best brick launch, over its planes per work item
-    if (ok && d.col_n > 0 && g.opt.precision == EMMA_PREC_MIXED && g.opt.column == 0 && shape_req < 0) {
+    // the column kernel against the best brick launch: its planes per work item, then
+    // (plain mixed variant) the warp-shuffle x sweep at the best depth against the
+    // shared-memory one, then balanced runs of column-planes against the items
+    if (ok && d.col_n > 0 && g.opt.column == 0 && shape_req < 0) {
+      DevLevel::Column &col = d.col[g.opt.precision == EMMA_PREC_MIXED];
+      auto timed = [&](int nz, int xs, int bal) {  // one warm-up, three timed
+        double ms = 0;
+        for (int rep = 0; rep < 4 && ok; rep++) {
+          ok = ck(cudaEventRecord(e0, g.stream), "event") &&
+               ck(launch_column(L, nz, nullptr, false, xs, bal), "column") && ck(cudaEventRecord(e1, g.stream), "event") &&
+               ck(cudaEventSynchronize(e1), "event");
+          float f = 0;
+          if (ok && rep > 0 && cudaEventElapsedTime(&f, e0, e1) == cudaSuccess) ms += f / 3.;
+        }
+        return ms;
+      };
       int best_nz = 0;
       double best_col = 0;
       for (int i = 0; i < 6 && ok; i++) {
         const int nz = kColNz[i];
-        d.col_sweep_ms[i] = 0;
+        col.sweep_ms[i] = 0;
         if (!column_nz_ok(d, nz)) continue;
-        double ms = 0;
-        for (int rep = 0; rep < 4 && ok; rep++) {  // one warm-up, three timed
-          ok = ck(cudaEventRecord(e0, g.stream), "event") && ck(launch_column(L, nz, nullptr, false, 0), "column") &&
-               ck(cudaEventRecord(e1, g.stream), "event") && ck(cudaEventSynchronize(e1), "event");
-          float f = 0;
-          if (ok && rep > 0 && cudaEventElapsedTime(&f, e0, e1) == cudaSuccess) ms += f / 3.;
-        }
-        d.col_sweep_ms[i] = ms;
+        const double ms = col.sweep_ms[i] = timed(nz, 0, 0);
         if (ok && (best_col == 0 || ms < best_col)) {
           best_col = ms;
           best_nz = nz;
         }
       }
-      // the warp-shuffle x sweep at the best depth against the shared-memory one
-      d.col_xs = 0;
-      d.col_xs_ms[0] = best_col;
-      d.col_xs_ms[1] = 0;
-      if (ok && best_nz > 0) {
-        double ms = 0;
-        for (int rep = 0; rep < 4 && ok; rep++) {
-          ok = ck(cudaEventRecord(e0, g.stream), "event") &&
-               ck(launch_column(L, best_nz, nullptr, false, 1), "column") && ck(cudaEventRecord(e1, g.stream), "event") &&
-               ck(cudaEventSynchronize(e1), "event");
-          float f = 0;
-          if (ok && rep > 0 && cudaEventElapsedTime(&f, e0, e1) == cudaSuccess) ms += f / 3.;
-        }
-        d.col_xs_ms[1] = ms;
+      col.xs = 0;
+      col.xs_ms[0] = best_col;
+      col.xs_ms[1] = 0;
+      if (ok && best_nz > 0 && g.opt.precision == EMMA_PREC_MIXED && column_variant() == 0u) {
+        const double ms = col.xs_ms[1] = timed(best_nz, 1, 0);
         if (ok && ms > 0 && ms < best_col) {
-          d.col_xs = 1;
+          col.xs = 1;
           best_col = ms;
         }
       }
-      // balanced runs of column-planes (the chosen x sweep) against the items
-      d.col_bal = 0;
-      d.col_bal_ms[0] = best_col;
-      d.col_bal_ms[1] = 0;
+      col.bal = 0;
+      col.bal_ms[0] = best_col;
+      col.bal_ms[1] = 0;
       if (ok && best_nz > 0) {
-        double ms = 0;
-        for (int rep = 0; rep < 4 && ok; rep++) {
-          ok = ck(cudaEventRecord(e0, g.stream), "event") &&
-               ck(launch_column(L, best_nz, nullptr, false, d.col_xs, 1), "column") &&
-               ck(cudaEventRecord(e1, g.stream), "event") && ck(cudaEventSynchronize(e1), "event");
-          float f = 0;
-          if (ok && rep > 0 && cudaEventElapsedTime(&f, e0, e1) == cudaSuccess) ms += f / 3.;
-        }
-        d.col_bal_ms[1] = ms;
+        const double ms = col.bal_ms[1] = timed(best_nz, col.xs, 1);
         if (ok && ms > 0 && ms < best_col) {
-          d.col_bal = 1;
+          col.bal = 1;
           best_col = ms;
         }
       }
-      d.col_nz = (ok && best_col > 0 && (best == 0 || best_col < best)) ? best_nz : 0;
+      col.nz = (ok && best_col > 0 && (best == 0 || best_col < best)) ? best_nz : 0;
     }
   }
   // undo the trial launches: corrections, completion counters, status
@@ -2000,31 +2010,31 @@ int emma_hydro_fused_job_log(int max, int *kinds, int *levels, double *release_u
 
 int emma_hydro_column_tuning(int level, int *planes, double *sweep_ms) {
   if (!level_ok(level)) return EMMA_ST_ARG;
-  const DevLevel &d = g.res.lev[level];
+  const DevLevel::Column &c = g.res.lev[level].col[g.opt.precision == EMMA_PREC_MIXED];
   if (planes) *planes = column_nz(level);
   if (sweep_ms)
-    for (int i = 0; i < 6; i++) sweep_ms[i] = d.col_sweep_ms[i];
+    for (int i = 0; i < 6; i++) sweep_ms[i] = c.sweep_ms[i];
   return 0;
 }
 
 int emma_hydro_column_xshfl(int level, int *xshfl, double *ms) {
   if (!level_ok(level)) return EMMA_ST_ARG;
-  const DevLevel &d = g.res.lev[level];
+  const DevLevel::Column &c = g.res.lev[level].col[g.opt.precision == EMMA_PREC_MIXED];
   if (xshfl) *xshfl = column_nz(level) > 0 ? column_xs(level) : 0;
   if (ms) {
-    ms[0] = d.col_xs_ms[0];
-    ms[1] = d.col_xs_ms[1];
+    ms[0] = c.xs_ms[0];
+    ms[1] = c.xs_ms[1];
   }
   return 0;
 }
 
 int emma_hydro_column_balanced(int level, int *balanced, double *ms) {
   if (!level_ok(level)) return EMMA_ST_ARG;
-  const DevLevel &d = g.res.lev[level];
+  const DevLevel::Column &c = g.res.lev[level].col[g.opt.precision == EMMA_PREC_MIXED];
   if (balanced) *balanced = column_nz(level) > 0 ? column_bal(level) : 0;
   if (ms) {
-    ms[0] = d.col_bal_ms[0];
-    ms[1] = d.col_bal_ms[1];
+    ms[0] = c.bal_ms[0];
+    ms[1] = c.bal_ms[1];
   }
   return 0;
 }

@@ -138,11 +138,6 @@ struct MathF64 {
     W[5] = rcp(W[0]);
     W[6] = root2(div_y(kGam * W[4], W[0], W[5]));
   }
-  // E of a face state (getE, src/hydro_utils.c:29)
-  static __device__ __forceinline__ double energy(const double W[7]) {
-    return over_g1(W[4]) + 0.5 * W[0] * (W[1] * W[1] + W[2] * W[2] + W[3] * W[3]);
-  }
-
   struct S1 { double d, u, p, a; };
 
   static __device__ double froot_prime(double p, const S1 &L, const S1 &R) {
@@ -165,7 +160,11 @@ struct MathF64 {
     return fL + fR + (R.u - L.u);
   }
   // findPressure (src/hydro_utils.c:680): rare fallback when the hybrid estimate is negative
-  static __device__ __noinline__ double pstar_exact(const S1 &L, const S1 &R, double *u, unsigned &st) {
+  // (everything by value: an address given to a call would keep the face's states and u* in
+  // local memory on the common path too)
+  struct StarState { double p, u; unsigned st; };
+  static __device__ __noinline__ StarState pstar_exact(S1 L, S1 R) {
+    unsigned st = 0;
     const double unsurz = (2.0 * kGam) / (kGam - 1.0);
     double pmin = fmin(L.p, R.p), pmax = fmax(L.p, R.p);
     double AL = 2. / ((kGam + 1.) * L.d), AR = 2. / ((kGam + 1.) * R.d);
@@ -193,8 +192,7 @@ struct MathF64 {
       if (froot(p, L, R, &u2) < kErrTol) break;
     }
     froot(p, L, R, &u2);
-    *u = u2;
-    return p;
+    return StarState{p, u2, st};
   }
 
   // x^5 = h + l to twice the working precision
@@ -205,14 +203,20 @@ struct MathF64 {
     l = __fma_rn(e4, x, __fma_rn(x4, x, -h));
   }
   // pow(x, z) for z = the double nearest 1/5, x > 0, to within 0.51 ulp (so nearly always the
-  // bits of a correctly rounded pow): an FP32 estimate w of x^(-1/5) good to 2^-20, one
-  // step of the series of (1 - h)^(-1/5) = 1 + h/5 + 3 h^2/25 + ..., h = 1 - x w^5, which
-  // leaves an error of an ulp or two, y = x w^4, and a Newton correction from the residual
-  // x - y^5 at twice the precision, plus y (z - 1/5) ln x.  Some 30 FP64 instructions
-  // where pow() takes a hundred or more.
-  static __device__ __forceinline__ double root5(double x) {
+  // bits of a correctly rounded pow), and iy = its reciprocal, rounded to nearest: an FP32
+  // estimate w of x^(-1/5) good to 2^-20, one step of the series of (1 - h)^(-1/5) =
+  // 1 + h/5 + 3 h^2/25 + ..., h = 1 - x w^5, which leaves an error of an ulp or two,
+  // y = x w^4, a Newton correction from the residual x - y^5 at twice the precision, plus
+  // y (z - 1/5) ln x; w is an ulp or two from 1/y, one Newton step rounds it.  Some 30
+  // FP64 instructions where pow() takes a hundred or more.
+  static constexpr double kZ = 1.1102230246251565e-17 * 0.6931471805599453;  // (z - 1/5) ln 2
+  static __device__ __forceinline__ double root5(double x, double &iy) {
     const float xf = (float)x;
-    if (!(xf > 1e-37f && xf < 1e37f)) return pow(x, 0.2);  // outside the estimate's range
+    if (!(xf > 1e-37f && xf < 1e37f)) {  // outside the estimate's range
+      const double y = pow(x, 0.2);
+      iy = 1. / y;
+      return y;
+    }
     const float lg = __log2f(xf);
     const double w0 = (double)exp2f(-0.2f * lg), v0 = w0 * w0;
     const double h = __fma_rn(-x, v0 * v0 * w0, 1.);
@@ -220,30 +224,42 @@ struct MathF64 {
     const double w2 = w * w, w4 = w2 * w2, y = x * w4;
     double y5, e5;
     pow5(y, y5, e5);
-    constexpr double kZ = 1.1102230246251565e-17 * 0.6931471805599453;  // (z - 1/5) ln 2
-    return y + __fma_rn((x - y5) - e5, 0.2 * w4, y * ((double)lg * kZ));
+    const double r = y + __fma_rn((x - y5) - e5, 0.2 * w4, y * ((double)lg * kZ));
+    iy = __fma_rn(w, __fma_rn(-r, w, 1.), w);
+    return r;
+  }
+  // pow(x, z) the same way from y, within some ulps of it
+  static __device__ __forceinline__ double root5_near(double x, double y) {
+    const float xf = (float)x;
+    if (!(xf > 1e-37f && xf < 1e37f)) return pow(x, 0.2);
+    double y5, e5, ix;
+    pow5(y, y5, e5);
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(ix) : "d"(x));
+    return y + __fma_rn((x - y5) - e5, 0.2 * y * ix, y * ((double)__log2f(xf) * kZ));
   }
 
   // Two-rarefaction star state of findPressure_Hybrid (src/hydro_utils.c:645-650),
   // {p*, u*}, the exponents 1/5 and 5 (a negative ratio, a vacuum-generating pair, gives
   // p* < 0 as pow() with an odd integer exponent does, and the exact solver replaces
-  // both).  Not inlined: it would crowd the instruction cache in every copy of the solver.
-  static __device__ __noinline__ double2 trrs(double aL, double aR, double uL, double uR, double pL, double pR) {
+  // both).  Inlined: a call from the middle of the solver saves the live state of the face
+  // in local memory (128^3 FP64 launch 0.493 ms against 0.445).
+  static __device__ __forceinline__ double2 trrs(double aL, double aR, double uL, double uR, double pL, double pR) {
     static_assert((kGam - 1.) / (2. * kGam) == 0.2 && (2. * kGam) / (kGam - 1.) == 5., "fifth roots need gamma = 5/3");
-    const double r = quot(aL + aR - (kGam - 1.) / 2. * (uR - uL), quot(aL, root5(pL)) + quot(aR, root5(pR)));
+    double iL, iR;
+    const double rL = root5(pL, iL), rR = root5(pR, iR);
+    const double r = quot(aL + aR - (kGam - 1.) / 2. * (uR - uL), div_y(aL, rL, iL) + div_y(aR, rR, iR));
     double h, l;
     pow5(r, h, l);
     const double pstar = h + l;
-    return make_double2(pstar, uL - over_g1(2. * aL) * (root5(quot(pstar, pL)) - 1.));
+    return make_double2(pstar, uL - over_g1(2. * aL) * (root5_near(quot(pstar, pL), r * iL) - 1.));
   }
 
-  // findPressure_Hybrid + speedestimate*_HLLC (src/hydro_utils.c:625,1264)
-  static __device__ __forceinline__ void speeds(const double WL[7], const double WR[7], int n, double &SL, double &SR,
+  // findPressure_Hybrid + speedestimate*_HLLC (src/hydro_utils.c:625,1264) of two states in
+  // the face's frame
+  static __device__ __forceinline__ void speeds(const double WL[7], const double WR[7], double &SL, double &SR,
                                                 double &ustar, unsigned &st) {
-    const double uLn = (n == 0) ? WL[1] : ((n == 1) ? WL[2] : WL[3]);
-    const double uRn = (n == 0) ? WR[1] : ((n == 1) ? WR[2] : WR[3]);
-    S1 L{WL[0], uLn, WL[4], WL[6]};
-    S1 R{WR[0], uRn, WR[4], WR[6]};
+    S1 L{WL[0], WL[1], WL[4], WL[6]};
+    S1 R{WR[0], WR[1], WR[4], WR[6]};
     double dbar = 0.5 * (L.d + R.d), abar = 0.5 * (L.a + R.a);
     double ppvrs = 0.5 * ((L.p + R.p) + (L.u - R.u) * dbar * abar);
     double pmax = fmax(L.p, R.p), pmin = fmin(L.p, R.p);
@@ -268,7 +284,12 @@ struct MathF64 {
       pstar = quot(GL * L.p + GR * R.p - (R.u - L.u), GL + GR);
       ustar = 0.5 * ((L.u + R.u) + (pstar - R.p) * GR - (pstar - L.p) * GL);
     }
-    if (pstar < 0) pstar = pstar_exact(L, R, &ustar, st);
+    if (pstar < 0) {
+      const StarState x = pstar_exact(L, R);
+      pstar = x.p;
+      ustar = x.u;
+      st |= x.st;
+    }
     if (pstar < 0) st |= kStNegPstar;
     double qL = 1., qR = 1.;
     if (!(pstar <= WL[4])) qL = root2(1. + (kGam + 1.) / (2. * kGam) * (quot(pstar, WL[4]) - 1.));
@@ -301,17 +322,20 @@ struct MathF64 {
     }
   }
 
-  // State rotated to the face frame: r = {d, u_n, u_t1, u_t2, p, E, |m|^2, 1/d},
-  // t1 < t2 the transverse axes in x,y,z order, |m|^2 summed in x,y,z order.
-  static __device__ __forceinline__ void rotate(const double W[7], int n, double r[8]) {
-    r[0] = W[0];
-    r[1] = (n == 0) ? W[1] : ((n == 1) ? W[2] : W[3]);
-    r[2] = (n == 0) ? W[2] : W[1];
-    r[3] = (n == 2) ? W[2] : W[3];
-    r[4] = W[4];
-    r[5] = energy(W);
+  // a + b + c of a face-frame triple (normal, t1, t2; t1 < t2 the transverse axes in x,y,z
+  // order) summed in x,y,z order: (n + t1) + t2 for the x and y axes (the first sum
+  // commutes), (t1 + t2) + n for z
+  static __device__ __forceinline__ double sum_xyz(double n, double t1, double t2, bool zax) {
+    return ((zax ? t2 : n) + t1) + (zax ? n : t2);
+  }
+  // r = {d, u_n, u_t1, u_t2, p, E, |m|^2, 1/d} of a state in the face's frame
+  // (E: getE, src/hydro_utils.c:29)
+  static __device__ __forceinline__ void frame_state(const double W[6], bool zax, double r[8]) {
+#pragma unroll
+    for (int i = 0; i < 5; i++) r[i] = W[i];
+    r[5] = over_g1(W[4]) + 0.5 * W[0] * sum_xyz(W[1] * W[1], W[2] * W[2], W[3] * W[3], zax);
     const double m0 = W[0] * W[1], m1 = W[0] * W[2], m2 = W[0] * W[3];
-    r[6] = m0 * m0 + m1 * m1 + m2 * m2;
+    r[6] = sum_xyz(m0 * m0, m1 * m1, m2 * m2, zax);
     r[7] = W[5];
   }
 
@@ -329,31 +353,38 @@ struct MathF64 {
     const double c = 0.5 * (kGam - 1.) * mn;
     f[4] = over_d(kGam * mn) * E - (IEEE ? c / (d * d) : div_yy(c, d, y)) * r[6];
   }
-  static __device__ __noinline__ void euler_ieee(const double r[8], double f[5]) { euler_quot<true>(r, f); }
+  struct Flux5 { double f[5]; };
+  static __device__ __noinline__ Flux5 euler_ieee(double d, double un, double t1, double t2, double E, double mm) {
+    const double r[8] = {d, un, t1, t2, 0., E, mm, 0.};
+    Flux5 x;
+    euler_quot<true>(r, x.f);
+    return x;
+  }
   static __device__ __forceinline__ void euler_rot(const double r[8], double f[5]) {
     euler_quot<false>(r, f);
     if (!isfinite(f[4])) {  // a quotient may have left div_y's range (every term of f enters f[4])
-      double t[8], u[5];
-      for (int i = 0; i < 8; i++) t[i] = r[i];
-      euler_ieee(t, u);
-      for (int i = 0; i < 5; i++) f[i] = u[i];
+      const Flux5 x = euler_ieee(r[0], r[1], r[2], r[3], r[5], r[6]);
+#pragma unroll
+      for (int i = 0; i < 5; i++) f[i] = x.f[i];
     }
   }
 
-  // HLLC flux across a face normal to axis n (src/hydro_utils.c:2055-2138),
-  // returned in x,y,z order: F = {mass, mom_x, mom_y, mom_z, energy}.
+  // HLLC flux across a face (src/hydro_utils.c:2055-2138) between two states in the
+  // face's frame {d, u_n, u_t1, u_t2, p, 1/d, a}; zax: the face is normal to z.
+  // F = {mass, mom_n, mom_t1, mom_t2, energy}.
   // du (dual-energy builds, optional): from the state Us of the branch taken (the
   // upwind or the star state), du[0] = Us.m_n / Us.d and du[1] = ebar =
   // Us.E - |Us.m|^2 / (2 Us.d) (src/hydro_utils.c:2126-2128).
   // xs, fx (tracer builds, optional): the centre fractions of the NT tracers,
   // xs[2 t] left and xs[2 t + 1] right, and their fluxes fx[t].
   template <int NT = 1>
-  static __device__ __forceinline__ void hllc(const double WL[7], const double WR[7], int n, double F[5],
-                                              unsigned &st, double *du = nullptr, const double *xs = nullptr,
-                                              double *fx = nullptr) {
+  static __device__ __forceinline__ void hllc_frame(const double WL[7], const double WR[7], bool zax, double G[5],
+                                                    unsigned &st, double *du = nullptr, const double *xs = nullptr,
+                                                    double *fx = nullptr) {
     double SL, SR, ustar;
-    speeds(WL, WR, n, SL, SR, ustar, st);
-    double G[5] = {0., 0., 0., 0., 0.};
+    speeds(WL, WR, SL, SR, ustar, st);
+#pragma unroll
+    for (int i = 0; i < 5; i++) G[i] = 0.;
     if (du != nullptr) du[0] = du[1] = 0.;
     if (fx != nullptr)
       for (int t = 0; t < NT; t++) fx[t] = 0.;
@@ -366,7 +397,7 @@ struct MathF64 {
       double W[7], r[8];
 #pragma unroll
       for (int i = 0; i < 6; i++) W[i] = left ? WL[i] : WR[i];
-      rotate(W, n, r);
+      frame_state(W, zax, r);
       euler_rot(r, G);
       const double d = r[0], un = r[1], E = r[5], y = r[7];
       if (upwind) {
@@ -395,17 +426,36 @@ struct MathF64 {
           }
         if (du != nullptr) {  // the star state: momenta in x,y,z order for the sum of squares
           const double ds = fact * 1., mn = fact * ustar, m1 = fact * r[2], m2 = fact * r[3];
-          const double mm = (n == 2) ? ((m1 * m1 + m2 * m2) + mn * mn) : ((mn * mn + m1 * m1) + m2 * m2);
+          const double mm = sum_xyz(mn * mn, m1 * m1, m2 * m2, zax);
           du[0] = mn / ds;
           du[1] = (fact * Es - 0.5 * mm / ds);
         }
       }
     }
+  }
+
+  // The same for states and flux in x,y,z order, the face normal to axis n.
+  template <int NT = 1>
+  static __device__ __forceinline__ void hllc(const double WL[7], const double WR[7], int n, double F[5], unsigned &st,
+                                              double *du = nullptr, const double *xs = nullptr, double *fx = nullptr) {
+    double l[7], r[7], G[5];
+    rotate(WL, n, l);
+    rotate(WR, n, r);
+    hllc_frame<NT>(l, r, n == 2, G, st, du, xs, fx);
     F[0] = G[0];
     F[1] = (n == 0) ? G[1] : G[2];
     F[2] = (n == 0) ? G[2] : ((n == 1) ? G[1] : G[3]);
     F[3] = (n == 2) ? G[1] : G[3];
     F[4] = G[4];
+  }
+  static __device__ __forceinline__ void rotate(const double W[7], int n, double r[7]) {
+    r[0] = W[0];
+    r[1] = (n == 0) ? W[1] : ((n == 1) ? W[2] : W[3]);
+    r[2] = (n == 0) ? W[2] : W[1];
+    r[3] = (n == 2) ? W[2] : W[3];
+    r[4] = W[4];
+    r[5] = W[5];
+    r[6] = W[6];
   }
 };
 
@@ -445,15 +495,23 @@ struct MathF32 {
   }
 
   // Face state toward face k from the predicted centre state X = W0 + Wt.
-  static __device__ __forceinline__ void face_px(const float X[5], const float Dax[5], int k, float W[7],
-                                                 unsigned &st) {
+  static __device__ __forceinline__ void face_px5(const float X[5], const float Dax[5], int k, float W[7],
+                                                  unsigned &st) {
     const float s = (k & 1) ? 0.5f : -0.5f;
 #pragma unroll
     for (int i = 0; i < 5; i++) W[i] = __fmaf_rn(s, Dax[i], X[i]);  // explicit: same rounding at every call site
     W[4] = fmaxf(W[4], (float)kPmin);
     if (W[0] < 0.f) st |= kStNegDensity;
+  }
+  // its 1/d and a
+  static __device__ __forceinline__ void face_finish(float W[7]) {
     W[5] = rcp(W[0]);
     W[6] = sqrtf(G * W[4] * W[5]);
+  }
+  static __device__ __forceinline__ void face_px(const float X[5], const float Dax[5], int k, float W[7],
+                                                 unsigned &st) {
+    face_px5(X, Dax, k, W, st);
+    face_finish(W);
   }
 
   static __device__ __forceinline__ float pstar_exact(float dL, float uL, float pL, float aL, float dR, float uR,

@@ -22,28 +22,17 @@ cudaError_t launch_step_f32(const StepArgs &a, unsigned variant, int groups, int
 
 int step_groups_f32(unsigned variant, int groups) { return step_groups_any<MathF32>(variant, groups); }
 
-// Column kernel of a complete periodic level (mixed path), two CTAs per SM; the
-// shared-memory or the warp-shuffle x sweep (ColumnArgs::xshfl).
-cudaError_t launch_column_f32(const ColumnArgs &a, cudaStream_t s) {
-  constexpr int kMaxDev = 64;
-  static bool attr_set[kMaxDev] = {false};  // the shared-memory limit is a per-device attribute
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (dev < 0 || dev >= kMaxDev) return cudaErrorInvalidDevice;
-  if (!attr_set[dev]) {
-    e = cudaFuncSetAttribute(column_kernel<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)col::kSmem);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(column_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)col::kSmem);
-    if (e != cudaSuccess) return e;
-    attr_set[dev] = true;
+// Column kernel of a complete level without split cells (launch flags `variant`: 0
+// plain, or one of kLaunchGrav, kLaunchDual, kLaunchTracer); the plain variant with
+// the shared-memory or the warp-shuffle x sweep (ColumnArgs::xshfl).
+cudaError_t launch_column_f32(const ColumnArgs &a, unsigned variant, cudaStream_t s) {
+  switch (variant) {
+    case 0u: return a.xshfl ? launch_column32<true, false, false, 0>(a, s) : launch_column32<false, false, false, 0>(a, s);
+    case kLaunchGrav: return launch_column32<false, true, false, 0>(a, s);
+    case kLaunchDual: return launch_column32<false, false, true, 0>(a, s);
+    case kLaunchTracer: return launch_column32<false, false, false, 1>(a, s);
+    default: return cudaErrorInvalidValue;
   }
-  if (a.nitems <= 0) return cudaSuccess;
-  if (a.xshfl)
-    column_kernel<2, true><<<a.nitems, col::kColThreads, col::kSmem, s>>>(a);
-  else
-    column_kernel<2, false><<<a.nitems, col::kColThreads, col::kSmem, s>>>(a);
-  return cudaGetLastError();
 }
 
 }  // namespace emma

@@ -137,23 +137,26 @@ struct BatchArgs {
   unsigned *ticket;     // work queue: [0] next item, [1] CTAs finished (reset by the last)
 };
 
-// A launch of the column kernel (column_kernel.cuh): one complete periodic level
-// without split cells, as columns of 16 x 16 cells marching through `nz` planes.
+// A launch of the column kernel (column_kernel.cuh): one complete level without
+// split cells, as columns of 16 x column_height() cells marching through `nz` planes.
 struct ColumnArgs {
   const LevelArgs *lv;  // the level's device slot: W, Wn, dt, dx are read at launch
   int L;
   const int *octidx;    // oct (list index) at every oct position, ((oz * n + oy) * n + ox)
   int n;                // octs per side
   int nz;               // cell planes per work item (even, divides 2n)
-  int ncol;             // columns per side (2n / 16)
-  int nitems;           // ncol * ncol * (2n / nz)
+  int ncol, ncoly;      // columns per side in x and y
+  int nitems;           // ncol * ncoly * (2n / nz)
   const int *gate;      // launch does nothing unless *gate != 0 (null: always)
   unsigned *status;
   unsigned long long *smax;  // [L]: max signal speed of the new state (bits of a double), or null
   int xshfl;            // x faces inside the column through warp shuffles (column_kernel.cuh XS)
   int balanced;         // nitems CTAs, each an equal run of the level's column-planes (nz unused)
+  int trans;            // transmissive x faces: bit 0 at -x, bit 1 at +x (else periodic)
 };
-constexpr int kColumnWidth = 16;  // cells per column side
+constexpr int kColumnWidth = 16;  // cells of a column in x
+constexpr int column_height(bool fp64) { return fp64 ? 8 : 16; }  // and in y
+constexpr int column_ctas(bool) { return 2; }                 // CTAs per SM of its launches
 
 constexpr int kWorkSlotShift = 24;
 constexpr int kMaxLevels = 32;
