@@ -8,13 +8,14 @@
 // caller passes the level state already on the device and receives dt; the
 // reduction's scratch is a fixed array inside this library.
 //
-// Scratch: g_dt_scratch, a file-scope __device__ array of kMaxBlocks + 1
-// 64-bit slots (128 KiB + 8 B) that every GPU which loads the library holds
-// until the process exits.  Slot b < kMaxBlocks receives the maximum signal
-// speed of block b, slot kMaxBlocks the maximum over the blocks.  Every slot a
-// call reads is written earlier in the same call, so nothing has to start at
-// zero; the array keeps the last call's values.  Calls whose kernels overlap on
-// the GPU (different streams, or several host threads) share the array and
+// Scratch: g_dt_scratch, a file-scope __device__ array of kMaxBlocks + 1 + kCounters
+// 64-bit slots (128.5 KiB) that every GPU which loads the library holds until the
+// process exits.  Slot b < kMaxBlocks receives the maximum signal speed of block b, slot
+// kMaxBlocks the maximum over the blocks; every one of these that a call reads is
+// written earlier in the same call.  The others count a call's finished blocks: call k
+// takes counter k mod kCounters and clears that of call k + kCounters / 2, so a counter
+// starts at zero whatever became of the call that used it before.  Calls whose kernels
+// overlap on the GPU (different streams, or several host threads) share the array and
 // race: serialise them on one stream.
 //
 // Host code only ever uses the array's device address, obtained once per device
@@ -38,15 +39,15 @@
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kCellsPerThread = 8;
 constexpr int kMaxBlocks = 16384;
-constexpr long long kCellsPerBlock = (long long)kThreads * kCellsPerThread;
-constexpr long long kMaxCells = kMaxBlocks * kCellsPerBlock;  // 33,554,432 cells (a 256^3 level is 16,777,216)
+constexpr int kCounters = 64;
+constexpr long long kMaxCells = 2048LL * kMaxBlocks;  // 33,554,432 cells (a 256^3 level is 16,777,216)
 constexpr int kMaxDevices = 64;
 
-static __device__ __align__(256) unsigned long long g_dt_scratch[kMaxBlocks + 1];
+static __device__ __align__(256) unsigned long long g_dt_scratch[kMaxBlocks + 1 + kCounters];
 
 std::atomic<unsigned long long *> g_scratch_addr[kMaxDevices];  // zero-initialised (static storage)
+std::atomic<unsigned> g_calls[kMaxDevices];
 
 __device__ __forceinline__ double block_max(double m) {
   __shared__ double part[kThreads / 32];
@@ -59,29 +60,44 @@ __device__ __forceinline__ double block_max(double m) {
   return m;
 }
 
-// per block: max over its cells of |v| + sqrt(gamma p / rho); W = 5 planes of n8 cells
-__global__ void __launch_bounds__(kThreads) dt_partial_kernel(const double *__restrict__ W, long long n8,
-                                                              unsigned long long *scratch) {
+// max over the cells of |v| + sqrt(gamma p / rho) -> scratch[kMaxBlocks]; W = 5 planes of
+// n8 cells.  One launch: each block leaves its maximum, the last to finish takes the
+// maximum over them.  A second launch for that cost as much as the whole reduction of a
+// small level (32^3: 30.6 us a call with two launches, 19.9 with one, most of it the
+// read-back).  Small levels take one cell a thread (latency; 128^3 32.9 -> 29.8 us), large
+// ones eight at a time (256^3 130 -> 127 us, 5.3 TB/s with the call's fixed cost).
+__global__ void __launch_bounds__(kThreads) dt_kernel(const double *__restrict__ W, long long n8, int per_thread,
+                                                      unsigned call, unsigned long long *scratch) {
   double m = 0.;
-  const long long base = blockIdx.x * kCellsPerBlock;
+  const long long base = (long long)blockIdx.x * kThreads * per_thread + threadIdx.x;
+  auto cell = [&](long long i) {
+    const double d = W[i], u = W[n8 + i], v = W[2 * n8 + i], w = W[3 * n8 + i], p = W[4 * n8 + i];
+    const double va = sqrt(u * u + v * v + w * w);
+    const double aa = sqrt((5. / 3.) * p / d);
+    m = fmax(m, va + aa);  // fmax drops NaN like the reference's FMAX
+  };
+  if (per_thread % 8 == 0 && base - threadIdx.x + (long long)per_thread * kThreads <= n8) {
+    for (int j = 0; j < per_thread; j += 8)
 #pragma unroll
-  for (int j = 0; j < kCellsPerThread; j++) {
-    const long long i = base + (long long)j * kThreads + threadIdx.x;
-    if (i < n8) {
-      const double d = W[i], u = W[n8 + i], v = W[2 * n8 + i], w = W[3 * n8 + i], p = W[4 * n8 + i];
-      const double va = sqrt(u * u + v * v + w * w);
-      const double aa = sqrt((5. / 3.) * p / d);
-      m = fmax(m, va + aa);  // fmax drops NaN like the reference's FMAX
-    }
+      for (int i = 0; i < 8; i++) cell(base + (long long)(j + i) * kThreads);
+  } else {
+    for (int j = 0; j < per_thread; j++)
+      if (base + (long long)j * kThreads < n8) cell(base + (long long)j * kThreads);
   }
   m = block_max(m);
-  if (threadIdx.x == 0) scratch[blockIdx.x] = (unsigned long long)__double_as_longlong(m);
-}
-
-// one block: max over the partials -> scratch[kMaxBlocks]
-__global__ void __launch_bounds__(kThreads) dt_final_kernel(unsigned long long *scratch, int nblocks) {
-  double m = 0.;
-  for (int b = threadIdx.x; b < nblocks; b += kThreads) m = fmax(m, __longlong_as_double((long long)scratch[b]));
+  __shared__ bool last;
+  if (threadIdx.x == 0) {
+    scratch[blockIdx.x] = (unsigned long long)__double_as_longlong(m);
+    unsigned long long *count = scratch + kMaxBlocks + 1;
+    if (blockIdx.x == 0) count[(call + kCounters / 2) % kCounters] = 0ULL;
+    __threadfence();
+    last = atomicAdd(count + call % kCounters, 1ULL) == gridDim.x - 1;
+  }
+  __syncthreads();  // also: block_max's shared memory is free again
+  if (!last) return;
+  __threadfence();
+  m = 0.;
+  for (int b = threadIdx.x; b < gridDim.x; b += kThreads) m = fmax(m, __longlong_as_double((long long)__ldcg(scratch + b)));
   m = block_max(m);
   if (threadIdx.x == 0) scratch[kMaxBlocks] = (unsigned long long)__double_as_longlong(m);
 }
@@ -111,9 +127,13 @@ extern "C" int emma_hydro_level_dt_noalloc(const double *d_state, long long ncel
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   double smax = 0.;
   if (ncells > 0) {
-    const int nblocks = (int)((ncells + kCellsPerBlock - 1) / kCellsPerBlock);
-    dt_partial_kernel<<<nblocks, kThreads, 0, s>>>(d_state, ncells, scratch);
-    dt_final_kernel<<<1, kThreads, 0, s>>>(scratch, nblocks);
+    // enough cells a thread to keep to 8 blocks an SM (148), a power of two up to 8; beyond
+    // 4096 blocks 16, or the counting of the blocks shows
+    int per = 1;
+    while (per < 8 && ncells > (long long)kThreads * per * 8 * 148) per *= 2;
+    if (ncells > (long long)kThreads * per * 4096) per = 16;
+    const int nblocks = (int)((ncells + (long long)kThreads * per - 1) / ((long long)kThreads * per));
+    dt_kernel<<<nblocks, kThreads, 0, s>>>(d_state, ncells, per, g_calls[dev].fetch_add(1u), scratch);
     if (cudaGetLastError() != cudaSuccess) return EMMA_ST_CUDA;
     unsigned long long bits = 0;
     if (cudaMemcpyAsync(&bits, scratch + kMaxBlocks, sizeof(bits), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
