@@ -175,7 +175,8 @@ def run_mine(args, rank, world):
                                                "column_x_sweep_shared_memory_warp_shuffle": [round(x, 4) for x in xms],
                                                "column_items_balanced": [round(x, 4) for x in bms]},
                                   "kernel": f"column ({planes} planes per item, {sweep})" if planes else "brick"}
-                kernels.add(f"column_kernel<2, {'true' if xs else 'false'}>" if planes else
+                kernels.add((f"column_kernel<{'true' if xs else 'false'}, ...>" if prec == PREC_MIXED else
+                             "column_fp64_kernel") if planes else
                             ("level_batch_kernel<MathF32>" if prec == PREC_MIXED else "level_batch_kernel<MathF64>"))
         init_states = {l: r.state(l) for l in levels}
         r.coarse_step(nsub=cfg.nsub)  # builds and instantiates the graph

@@ -771,7 +771,8 @@ int column_bal(int L) {
   return g.opt.column > 0 ? 0 : g.res.lev[L].col[g.opt.precision == EMMA_PREC_MIXED].bal;
 }
 
-cudaError_t launch_column(int L, int nz, const int *gate, bool fuse_cfl, int xs = -1, int bal = -1) {
+// end: the launch also ends the step (schedule.h batch_end)
+cudaError_t launch_column(int L, int nz, const int *gate, bool fuse_cfl, int xs = -1, int bal = -1, bool end = false) {
   const DevLevel &d = g.res.lev[L];
   const bool fp64 = g.opt.precision != EMMA_PREC_MIXED;
   ColumnArgs c;
@@ -793,6 +794,7 @@ cudaError_t launch_column(int L, int nz, const int *gate, bool fuse_cfl, int xs 
   c.status = g.d_status;
   c.smax = fuse_cfl ? g.d_S->smax_next : nullptr;
   c.xshfl = xs >= 0 ? xs : column_xs(L);
+  c.end = end ? g.d_S : nullptr;
   c.trans = ((g.res.host.trans & EMMA_TRANS_XM) ? 1 : 0) | ((g.res.host.trans & EMMA_TRANS_XP) ? 2 : 0);
   return fp64 ? launch_column_fp64(c, column_variant(), g.stream) : launch_column_f32(c, column_variant(), g.stream);
 }
@@ -949,6 +951,16 @@ bool emit_coarse_step(int nsub) {
   SchedState *S = g.d_S;
   const int lc = t.lcoarse, lf = finest_level();
   if (nsub == 1 || lf == lc) {
+    if (lf == lc && column_nz(lc) > 0) {
+      // one level on the column kernel: CFL, dt and binding in one launch, the level and the
+      // end of the step in the other (four launches cost 4.7 us more than the kernel's own
+      // 23 us a step on a 32^3 box)
+      const long long blocks = std::max(1LL, std::min((t.lev[lc].n8 + 255) / 256, 4LL * g.nsm));
+      k_cfl_begin<<<(unsigned)blocks, 256, 0, g.stream>>>(S, t.d_lv, g.d_done, lc);
+      g.kernel_launches++;
+      return ck(cudaGetLastError(), "schedule kernel") &&
+             ck(launch_column(lc, column_nz(lc), nullptr, true, -1, -1, true), "column launch");
+    }
     // one dt for every level: CFL per level (from the previous launch's fused maxima, or a
     // reduction kernel where the state was set from the host), then all levels in one launch
     for (int L = lc; L <= lf; L++) {

@@ -352,6 +352,8 @@ __global__ void __launch_bounds__((Col64<DUAL, NTR>::kThreads), column_ctas(true
   if (a.smax != nullptr && threadIdx.x < kInt / 32 && U.wmax[threadIdx.x] > 0.)  // after the last step's barrier
     atomicMax(a.smax + a.L, (unsigned long long)__double_as_longlong(U.wmax[threadIdx.x]));
   if (st) atomicOr(a.status, st);
+  // every thread has read the level's slot
+  if (a.end != nullptr && threadIdx.x == 0) batch_end_by_last(a.end, const_cast<LevelArgs *>(a.lv) - a.L);
 }
 
 namespace {  // internal linkage, as the other launchers

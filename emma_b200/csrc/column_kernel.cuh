@@ -47,7 +47,7 @@
 #pragma once
 #include <type_traits>
 #include "hydro_math.cuh"
-#include "plan_types.h"
+#include "schedule.h"
 
 namespace emma {
 
@@ -179,10 +179,9 @@ __device__ __forceinline__ void column_segments(const ColumnArgs &a, const F &se
 // Bound by instruction issue (53% of cycles at 128^3, 17 warps an SM: 42.6 warp
 // instructions a cell, FP32 pipe 40% of them, minima, compares and selects 31%), not by
 // memory (70 bytes a cell of DRAM traffic).  Measured a launch, against slopes and all
-// three axes through shared memory and the brick kernel: 256^3 1.07 ms (1.20, 1.66), 128^3
-// 0.151 ms (0.174, 0.224); against the brick kernel, dual energy 0.181 ms (0.248),
-// gravity 0.183 ms (0.245), tracer 0.184 ms (0.262) at 128^3, 64^3 with transmissive x
-// 0.033 ms (0.044).
+// three axes through shared memory and the brick kernel: 256^3 0.99 ms (1.20, 1.66), 128^3
+// 0.141 ms (0.174, 0.224); against the brick kernel, dual energy 0.158 ms (0.248) at
+// 128^3, 64^3 with transmissive x 0.031 ms (0.044).
 template <bool XS, bool GRAV, bool DUAL, int NTR>
 __global__ void __launch_bounds__((Col32<DUAL, NTR>::kThreads), column_ctas(false)) column_kernel(const ColumnArgs a) {
   using M = MathF32;
@@ -425,9 +424,6 @@ __global__ void __launch_bounds__((Col32<DUAL, NTR>::kThreads), column_ctas(fals
     for (int z = z0 - 1; z <= z1; z++) {
       // ---------------------------------------------------------------- A
       const bool xy = z >= z0 && z < z1;  // the halo planes close z faces only
-      const bool upd = interior && z > z0;
-      long long gu = 0;
-      double qu[5];  // FP64 state of plane z-1 (mixed path: again from L2, staged three planes ago)
       R Fn[5] = {}, dn[2] = {}, fn[NT] = {};  // the -z flux of plane z
       if (cell) {
         R D[3][5], Wt[5], X[5], gk[3] = {(R)0, (R)0, (R)0};
@@ -485,10 +481,6 @@ __global__ void __launch_bounds__((Col32<DUAL, NTR>::kThreads), column_ctas(fals
         R zl[5], zh[5];
         face(std::integral_constant<int, 4>{}, zl);
         face(std::integral_constant<int, 5>{}, zh);
-        if (upd) {  // lands while the z face is solved
-          gu = gidx(oct_at(oxy1, z - 1), cxy1, z - 1);
-          load5(gu, qu);
-        }
         if (interior && z >= z0) {
           R xs[2 * NT];
 #pragma unroll
@@ -516,7 +508,15 @@ __global__ void __launch_bounds__((Col32<DUAL, NTR>::kThreads), column_ctas(fals
           tc[t] = tn[t];
         }
       }
-      if (upd) update(gu, qu, Fz, Fn, dz, dn, fz, fn);
+      if (interior && z > z0) {
+        // the FP64 state of plane z-1 again, from L2: loaded here and not ahead of the z
+        // face, whose solve would carry its 10 registers (128^3 0.151 against 0.146 ms, dual
+        // energy 0.180 against 0.158)
+        const long long gu = gidx(oct_at(oxy1, z - 1), cxy1, z - 1);
+        double qu[5];
+        load5(gu, qu);
+        update(gu, qu, Fz, Fn, dz, dn, fz, fn);
+      }
       if (interior) {
 #pragma unroll
         for (int v = 0; v < 5; v++) Fz[v] = Fn[v];
@@ -529,16 +529,34 @@ __global__ void __launch_bounds__((Col32<DUAL, NTR>::kThreads), column_ctas(fals
       }
       __syncthreads();
       // ---------------------------------------------------------------- B
-      // the loads of plane z+2 land while the x faces are solved, those of its second
-      // column while the y faces are; its slot held plane z, read before the barrier
+      // The loads of plane z+2 land while the y faces are solved (dual energy: from the x
+      // faces on, those of the second column while the y faces are).  Its slot held plane
+      // z, read before the barrier.  Ahead of the x faces their 10 registers cost the plain
+      // variant more than the latency they hide (128^3 0.146 against 0.141 ms, 256^3 1.031
+      // against 0.992; dual energy 0.158 against 0.160 the other way round).
       const bool next = cell && z < z1, next2 = conv2 && z + 1 < z1;
       double q[5];
       long long gi = 0;
-      if (next) {
-        gi = gidx(on1, cxy1, z + 2);
-        load5(gi, q);
-        on1 = oct_at(oxy1, z + 3);
-      }
+      auto load_next = [&]() {
+        if (next) {
+          gi = gidx(on1, cxy1, z + 2);
+          load5(gi, q);
+          on1 = oct_at(oxy1, z + 3);
+        }
+      };
+      auto stage_next = [&]() {
+        if (next) {
+          stage(z + 2, rp, q, qn);
+          fractions_of(gi, q[0], tn);
+        }
+      };
+      auto load_next2 = [&]() {
+        if (next2) {
+          load5(gidx(on2, cxy2, z + 2), q);
+          on2 = oct_at(oxy2, z + 3);
+        }
+      };
+      if constexpr (DUAL) load_next();
       R F[5], du[2] = {}, fx[NT], xs[2 * NT], L5[5], R5[5];
       auto keep = [&](unsigned char *sF, R *sE, int n, int e) {
         V::st(sF, n, e, F);
@@ -582,13 +600,11 @@ __global__ void __launch_bounds__((Col32<DUAL, NTR>::kThreads), column_ctas(fals
         solve(D0{}, L5, R5, F, du, xs, fx);
         keep(sFX, sEX, C::kSX, e);
       }
-      if (next) {
-        stage(z + 2, rp, q, qn);
-        fractions_of(gi, q[0], tn);
-      }
-      if (next2) {
-        load5(gidx(on2, cxy2, z + 2), q);
-        on2 = oct_at(oxy2, z + 3);
+      if constexpr (DUAL) {
+        stage_next();
+        load_next2();
+      } else {
+        load_next();
       }
       if constexpr (GRAV) {
         if (next) {  // the acceleration at plane z+1
@@ -603,6 +619,10 @@ __global__ void __launch_bounds__((Col32<DUAL, NTR>::kThreads), column_ctas(fals
         solve(D1{}, L5, ylo, F, du, xs, fx);
         keep(sFY, sEY, C::kSY, ey);
       }
+      if constexpr (!DUAL) {
+        stage_next();
+        load_next2();
+      }
       if (next2) {
         R x[5];
         stage(z + 2, hp, q, x);
@@ -615,6 +635,8 @@ __global__ void __launch_bounds__((Col32<DUAL, NTR>::kThreads), column_ctas(fals
   if (a.smax != nullptr && interior && (tid & 31) == 0 && wmax > 0.)
     atomicMax(a.smax + a.L, (unsigned long long)__double_as_longlong(wmax));
   if (st) atomicOr(a.status, st);
+  // every thread has read the level's slot
+  if (a.end != nullptr && threadIdx.x == 0) batch_end_by_last(a.end, const_cast<LevelArgs *>(a.lv) - a.L);
 }
 
 // The launchers have internal linkage, as the level kernel's (level_kernel.cuh): the

@@ -153,6 +153,7 @@ struct ColumnArgs {
   int xshfl;            // x faces inside the column through warp shuffles (column_kernel.cuh XS)
   int balanced;         // nitems CTAs, each an equal run of the level's column-planes (nz unused)
   int trans;            // transmissive x faces: bit 0 at -x, bit 1 at +x (else periodic)
+  struct SchedState *end;  // the last CTA ends the step (schedule.h batch_end), or null
 };
 constexpr int kColumnWidth = 16;  // cells of a column in x
 constexpr int column_height(bool fp64) { return fp64 ? 8 : 16; }  // and in y

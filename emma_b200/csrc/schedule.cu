@@ -66,7 +66,7 @@ __global__ void k_clear(double *p, long long n, const int *gate) {
 // overwritten by the finer level's, src/advanceamr.c:808-858).  All levels then
 // go through one launch, finest first, each level's update waiting for the finer
 // level's (corrections, new state for split-cell averaging).
-__global__ void k_batch_begin(SchedState *S, LevelArgs *lv, unsigned *done) {
+static __device__ __forceinline__ void batch_begin(SchedState *S, LevelArgs *lv, unsigned *done) {
   const int lc = S->lcoarse, lm = S->lmax;
   double *adt = S->adt;
   const double tloc = S->tsim;
@@ -101,21 +101,29 @@ __global__ void k_batch_begin(SchedState *S, LevelArgs *lv, unsigned *done) {
   S->gate_all = 1;
 }
 
-__global__ void k_batch_end(SchedState *S, LevelArgs *lv) {
-  const int lc = S->lcoarse, lm = S->lmax;
-  for (int L = lc; L <= lm; L++) {
-    if (lv[L].noct == 0) break;
-    double *t = lv[L].W;
-    lv[L].W = lv[L].Wn;
-    lv[L].Wn = t;
-    lv[L].wait_slot = -1;
-    S->updates += lv[L].leaf;
-    S->fresh[L] = 1;
-    S->stale[L] = 0;
-    S->azall[L] = 1;
+__global__ void k_batch_begin(SchedState *S, LevelArgs *lv, unsigned *done) { batch_begin(S, lv, done); }
+
+// The CFL reduction of a tree's only level and batch_begin in one launch.  The state of
+// all steps but the first after a host-side change was written by the level kernel, which
+// left its maximum: then the first block goes straight on.  Otherwise the last block of
+// the reduction does.
+__global__ void k_cfl_begin(SchedState *S, LevelArgs *lv, unsigned *done, int L) {
+  if (!S->stale[L]) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) batch_begin(S, lv, done);
+    return;
   }
-  S->tsim += S->adt[lc - 1];
+  cfl_block(lv[L].W, 8LL * lv[L].noct, &S->smax[L]);
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(&S->ticket[1], 1u) == gridDim.x - 1) {
+      S->ticket[1] = 0u;
+      __threadfence();
+      batch_begin(S, lv, done);
+    }
+  }
 }
+
+__global__ void k_batch_end(SchedState *S, LevelArgs *lv) { batch_end(S, lv); }
 
 // ------------------------------------------------ subcycled (Advance_level)
 // One loop iteration `it` of Advance_level(L): the gate of this iteration.

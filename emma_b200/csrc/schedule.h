@@ -62,11 +62,62 @@ struct StepJobRecord {
 };
 constexpr unsigned kStepJobLog = 256;
 
+// The CFL reduction of a level (src/advanceamr.c:122-128) by a grid of 256-thread blocks:
+// this block's share of the cells, the maximum added to *out (bits of a non-negative
+// double, which order like the numbers).  For units built with -fmad=false.
+static __device__ __forceinline__ void cfl_block(const double *__restrict__ W, long long n8, unsigned long long *out) {
+  double m = 0.;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n8; i += (long long)gridDim.x * blockDim.x) {
+    const double d = W[i], u = W[n8 + i], v = W[2 * n8 + i], w = W[3 * n8 + i], p = W[4 * n8 + i];
+    const double va = sqrt(u * u + v * v + w * w);
+    const double aa = sqrt((5. / 3.) * p / d);
+    const double s = va + aa;
+    m = fmax(m, s);  // fmax drops NaN like the reference's FMAX
+  }
+  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+  __shared__ double sm[32];
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    m = (threadIdx.x < (blockDim.x >> 5)) ? sm[threadIdx.x] : 0.;
+    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (threadIdx.x == 0) atomicMax(out, (unsigned long long)__double_as_longlong(m));
+  }
+}
+
+// The end of a step that advanced every level once: buffers swapped, counters, time.
+static __device__ __forceinline__ void batch_end(SchedState *S, LevelArgs *lv) {
+  const int lc = S->lcoarse, lm = S->lmax;
+  for (int L = lc; L <= lm; L++) {
+    if (lv[L].noct == 0) break;
+    double *t = lv[L].W;
+    lv[L].W = lv[L].Wn;
+    lv[L].Wn = t;
+    lv[L].wait_slot = -1;
+    S->updates += lv[L].leaf;
+    S->fresh[L] = 1;
+    S->stale[L] = 0;
+    S->azall[L] = 1;
+  }
+  S->tsim += S->adt[lc - 1];
+}
+
+// ... run by the last block of a launch to finish (one thread of each block calls this,
+// after the block's last access to the level slots); S->ticket[1] counts the blocks.
+static __device__ __forceinline__ void batch_end_by_last(SchedState *S, LevelArgs *lv) {
+  __threadfence();
+  if (atomicAdd(&S->ticket[1], 1u) == gridDim.x - 1) {
+    S->ticket[1] = 0u;
+    batch_end(S, lv);
+  }
+}
+
 __global__ void k_set_args(LevelArgs *lv, int slot, LevelArgs a);
 __global__ void k_bind_level(LevelArgs *lv, int L, int lcoarse, int lmax, double dt);
 __global__ void k_swap_level(LevelArgs *lv, int L, const int *gate);
 __global__ void k_clear(double *p, long long n, const int *gate);
 __global__ void k_batch_begin(SchedState *S, LevelArgs *lv, unsigned *done);
+__global__ void k_cfl_begin(SchedState *S, LevelArgs *lv, unsigned *done, int L);
 __global__ void k_batch_end(SchedState *S, LevelArgs *lv);
 __global__ void k_sub_begin(SchedState *S, int L, int it);
 __global__ void k_sub_dt(SchedState *S, int L);

@@ -17,7 +17,7 @@ def options(precision=PREC_FP64, trans=0, cfl=0.85, device=0, use_graph=True, ti
     """tile_octs: 0 = brick shape autotuned per level at upload, 32 = 4x4x2-oct
     bricks, 8 = 2x2x2-oct bricks (four per tile).  gravity: the -DWGRAV coupling
     (forces from ResidentHydro.set_force).  dual: the -DDUAL_E tracked internal energy.
-    column (mixed path, complete periodic levels without split cells): 0 = the
+    column (complete levels without split cells, periodic or transmissive in x): 0 = the
     autotuner picks the column kernel or the brick kernel, -1 = brick kernel only,
     n > 0 = column kernel with n cell planes per work item.  fused (subcycled
     coarse steps on the graph): "auto" = the autotuner picks the fused kernel (one

@@ -73,11 +73,13 @@ struct EmmaHydroOptions {
                            flux and a p div(u) term, and the pressure comes from it unless
                            E - Ekin is resolved (src/hydro_utils.c:45-49, 2126-2129,
                            3164-3182).  Drop-in and resident modes. */
-  int column;           /* mixed precision, resident complete periodic levels without split
-                           cells (plain variant): 0 = the autotuner picks the column kernel
-                           (16 x 16-cell columns marching through z) or the brick kernel,
-                           -1 = brick kernel only, n > 0 = column kernel with n cell planes
-                           per work item (even, dividing the level's cells per side) */
+  int column;           /* resident complete levels without split cells, periodic or transmissive
+                           in x (plain, gravity, dual energy or one tracer): 0 = the autotuner
+                           picks the column kernel (columns of cells marching through z) or the
+                           brick kernel, -1 = brick kernel only, n > 0 = column kernel with n cell
+                           planes per work item (even, dividing the level's cells per side).  A
+                           forced brick shape (tile_octs) means the brick kernel, except on the
+                           plain mixed path of periodic levels */
   int fused_step;       /* subcycled coarse steps of a resident tree on the CUDA graph: one
                            persistent kernel per coarse step that runs the whole level recursion
                            (plain, dual-energy and tracer trees without gravity or transmissive
@@ -86,7 +88,7 @@ struct EmmaHydroOptions {
                            timed over five coarse steps from a snapshot of the state, which is
                            then restored), -1 = separate launches, k > 0 = fused with k tile
                            groups per CTA (as many as fit if k is not built) */
-  int column_xshfl;     /* x sweep of the column kernel: the faces inside a 16-cell row solved
+  int column_xshfl;     /* x sweep of the plain mixed column kernel: the faces inside a 16-cell row solved
                            from the left cell's face state passed up a lane by a warp shuffle
                            (1) or read from shared memory (-1); 0 = the faster of the two at
                            the autotuned depth (shared memory when `column` forces a depth) */
