@@ -1002,6 +1002,8 @@ bool emit_coarse_step(int nsub) {
     a.status = g.d_status;
     a.wait_limit = g.wait_limit;
     a.lfine = lf;
+    a.shapes = 0;
+    for (int L = lc; L <= lf; L++) a.shapes |= 1u << t.lev[L].shape;
     a.jobt = g.d_jobt;
     const unsigned variant = (g.opt.dual_energy ? kLaunchDual : 0u) | kLaunchTracers;
     const cudaError_t e = (g.opt.precision == EMMA_PREC_MIXED)

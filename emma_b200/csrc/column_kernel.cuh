@@ -179,8 +179,8 @@ __device__ __forceinline__ void column_segments(const ColumnArgs &a, const F &se
 // Bound by instruction issue (53% of cycles at 128^3, 17 warps an SM: 42.6 warp
 // instructions a cell, FP32 pipe 40% of them, minima, compares and selects 31%), not by
 // memory (70 bytes a cell of DRAM traffic).  Measured a launch, against slopes and all
-// three axes through shared memory and the brick kernel: 256^3 0.99 ms (1.20, 1.66), 128^3
-// 0.141 ms (0.174, 0.224); against the brick kernel, dual energy 0.158 ms (0.248) at
+// three axes through shared memory and the brick kernel: 256^3 0.975 ms (1.20, 1.66), 128^3
+// 0.139 ms (0.174, 0.224); against the brick kernel, dual energy 0.159 ms (0.248) at
 // 128^3, 64^3 with transmissive x 0.031 ms (0.044).
 template <bool XS, bool GRAV, bool DUAL, int NTR>
 __global__ void __launch_bounds__((Col32<DUAL, NTR>::kThreads), column_ctas(false)) column_kernel(const ColumnArgs a) {
@@ -510,8 +510,8 @@ __global__ void __launch_bounds__((Col32<DUAL, NTR>::kThreads), column_ctas(fals
       }
       if (interior && z > z0) {
         // the FP64 state of plane z-1 again, from L2: loaded here and not ahead of the z
-        // face, whose solve would carry its 10 registers (128^3 0.151 against 0.146 ms, dual
-        // energy 0.180 against 0.158)
+        // face, whose solve would carry its 10 registers (128^3 0.151 against 0.139 ms, dual
+        // energy 0.180 against 0.159)
         const long long gu = gidx(oct_at(oxy1, z - 1), cxy1, z - 1);
         double qu[5];
         load5(gu, qu);
@@ -529,34 +529,16 @@ __global__ void __launch_bounds__((Col32<DUAL, NTR>::kThreads), column_ctas(fals
       }
       __syncthreads();
       // ---------------------------------------------------------------- B
-      // The loads of plane z+2 land while the y faces are solved (dual energy: from the x
-      // faces on, those of the second column while the y faces are).  Its slot held plane
-      // z, read before the barrier.  Ahead of the x faces their 10 registers cost the plain
-      // variant more than the latency they hide (128^3 0.146 against 0.141 ms, 256^3 1.031
-      // against 0.992; dual energy 0.158 against 0.160 the other way round).
+      // the loads of plane z+2 land while the x faces are solved, those of its second
+      // column while the y faces are; its slot held plane z, read before the barrier
       const bool next = cell && z < z1, next2 = conv2 && z + 1 < z1;
       double q[5];
       long long gi = 0;
-      auto load_next = [&]() {
-        if (next) {
-          gi = gidx(on1, cxy1, z + 2);
-          load5(gi, q);
-          on1 = oct_at(oxy1, z + 3);
-        }
-      };
-      auto stage_next = [&]() {
-        if (next) {
-          stage(z + 2, rp, q, qn);
-          fractions_of(gi, q[0], tn);
-        }
-      };
-      auto load_next2 = [&]() {
-        if (next2) {
-          load5(gidx(on2, cxy2, z + 2), q);
-          on2 = oct_at(oxy2, z + 3);
-        }
-      };
-      if constexpr (DUAL) load_next();
+      if (next) {
+        gi = gidx(on1, cxy1, z + 2);
+        load5(gi, q);
+        on1 = oct_at(oxy1, z + 3);
+      }
       R F[5], du[2] = {}, fx[NT], xs[2 * NT], L5[5], R5[5];
       auto keep = [&](unsigned char *sF, R *sE, int n, int e) {
         V::st(sF, n, e, F);
@@ -600,11 +582,13 @@ __global__ void __launch_bounds__((Col32<DUAL, NTR>::kThreads), column_ctas(fals
         solve(D0{}, L5, R5, F, du, xs, fx);
         keep(sFX, sEX, C::kSX, e);
       }
-      if constexpr (DUAL) {
-        stage_next();
-        load_next2();
-      } else {
-        load_next();
+      if (next) {
+        stage(z + 2, rp, q, qn);
+        fractions_of(gi, q[0], tn);
+      }
+      if (next2) {
+        load5(gidx(on2, cxy2, z + 2), q);
+        on2 = oct_at(oxy2, z + 3);
       }
       if constexpr (GRAV) {
         if (next) {  // the acceleration at plane z+1
@@ -618,10 +602,6 @@ __global__ void __launch_bounds__((Col32<DUAL, NTR>::kThreads), column_ctas(fals
         fractions(tly);
         solve(D1{}, L5, ylo, F, du, xs, fx);
         keep(sFY, sEY, C::kSY, ey);
-      }
-      if constexpr (!DUAL) {
-        stage_next();
-        load_next2();
       }
       if (next2) {
         R x[5];

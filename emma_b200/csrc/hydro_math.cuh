@@ -508,12 +508,6 @@ struct MathF32 {
     W[5] = rcp(W[0]);
     W[6] = sqrtf(G * W[4] * W[5]);
   }
-  static __device__ __forceinline__ void face_px(const float X[5], const float Dax[5], int k, float W[7],
-                                                 unsigned &st) {
-    face_px5(X, Dax, k, W, st);
-    face_finish(W);
-  }
-
   static __device__ __forceinline__ float pstar_exact(float dL, float uL, float pL, float aL, float dR, float uR,
                                                    float pR, float aR, float *u) {
     // Newton iteration on the exact two-rarefaction/shock function (Toro sec. 4.3)

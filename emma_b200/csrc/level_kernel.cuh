@@ -217,8 +217,7 @@ struct TileSmem {
   static constexpr size_t off_args = kTabBytes;                                // LevelArgs of the tile's level
   // per-slot descriptors
   static constexpr size_t off_key = a16(off_args + sizeof(LevelArgs));         // u32 [kDB][NS]
-  static constexpr size_t off_ob = a16(off_key + 4 * kDB * NS);                // i32 [kDB][NS] source offset
-  static constexpr size_t off_sf = a16(off_ob + 4 * kDB * NS);                 // u8  [kDB][NS] slot flags
+  static constexpr size_t off_sf = a16(off_key + 4 * kDB * NS);                // u8  [kDB][NS] slot flags
   static constexpr size_t off_spm = a16(off_sf + kDB * NS);                    // u8  [kDB][NS] split mask (cell order)
   static constexpr size_t off_cmk = a16(off_spm + kDB * NS);                   // u8  [kDB][NS] cell map
   static constexpr size_t off_st = a16(off_cmk + kDB * NS);                    // u8  [NBOX] cell flags
@@ -230,10 +229,9 @@ struct TileSmem {
   static constexpr int kMG = kF64 ? 6 : 5;
   static constexpr size_t off_M = a16(off_Wp + sizeof(R) * NBOX);
   static constexpr size_t off_Mp = off_M + sizeof(R) * 4 * kMG * kThreads;
-  // ring face states: FP32 R4 [2][NRING] (d,u,v,w | p,1/d,a); FP64 R4 [NRING] + R [NRING]
-  // (d,u,v,w | p: a and E are recomputed by the consumer)
+  // ring face states: R4 [NRING] + R [NRING] (d,u,v,w | p; 1/d and a are the consumer's)
   static constexpr size_t off_HS = a16(off_Mp + (kF64 ? sizeof(R) * kThreads : 0));
-  static constexpr size_t off_end = a16(off_HS + (kF64 ? sizeof(R) * 5 * NRING : sizeof(R) * 4 * 2 * NRING));
+  static constexpr size_t off_end = a16(off_HS + sizeof(R) * 5 * NRING);
   // face fluxes reuse the staged box, dead after reconstruction
   static constexpr size_t off_F = off_W;                                // R4 [NFS]
   static constexpr size_t off_F1 = a16(off_F + sizeof(R) * 4 * NFS);    // R  [NFS]
@@ -278,7 +276,6 @@ __device__ __forceinline__ void level_tile(const BatchArgs &Bt, const LevelArgs 
   constexpr int NS = SM::NS, NRING = SM::NRING;
   using V = Q4<R>;
   uint32_t *sKey = reinterpret_cast<uint32_t *>(smem + SM::off_key) + cur * NS;
-  int *sOb = reinterpret_cast<int *>(smem + SM::off_ob) + cur * NS;
   uint8_t *sSf = smem + SM::off_sf + cur * NS;
   uint8_t *sSpm = smem + SM::off_spm + cur * NS;
   uint8_t *sCmk = smem + SM::off_cmk + cur * NS;
@@ -340,25 +337,22 @@ __device__ __forceinline__ void level_tile(const BatchArgs &Bt, const LevelArgs 
   };
 
   // ------------------------------------------------------------------ P0
-  // per slot: key, source offset, flags, split mask in cell order, cell map
+  // per slot: key, flags, split mask in cell order, cell map
   // (0: cell c of an oct, 1: an injected cell, 2+k: mirror across face k);
   // `raw` is the split byte of a real or ghost slot's oct
   auto build = [&](int i, uint32_t key, uint8_t raw, uint32_t mask, int off) {
     const int nb = i / G::kSlots, s = i - nb * G::kSlots;
     uint8_t sf = 0, spm = 0, cmk = 0;
-    int ob = 0;
     if (key != kKeyNone) {
-      const uint32_t kind = key >> 28, idx = key & 0x0FFFFFFFu;
+      const uint32_t kind = key >> 28;
       sf = kFPresent;
       if (kind == kKeyReal) {
-        ob = 8 * (int)idx;
         spm = raw;
         const uint8_t bit = sBit[s];
         if (bit != 255 && ((mask >> (nb * G::kOcts + bit)) & 1)) sf |= kFTile;
       } else if (kind == kKeyInj) {
         cmk = 1;
         if (A.Wc != nullptr) {
-          ob = (int)idx;
           sf |= kFInj;
         } else {
           st |= kStTree;  // plan/launch mismatch: never read through a null level
@@ -367,13 +361,11 @@ __device__ __forceinline__ void level_tile(const BatchArgs &Bt, const LevelArgs 
         if (A.wv_inject) {  // gravity build: the coarse cell injected (its force is interpolated)
           cmk = 1;
           if (A.Wc != nullptr && A.vcell != nullptr) {
-            ob = __ldg(A.vcell + 7 * (size_t)idx);
             sf |= kFInj;
           } else {
             st |= kStTree;
           }
         } else if (A.Wv != nullptr) {  // 8 interpolated sub-cells, laid out like an oct
-          ob = 8 * (int)idx;
           sf |= kFInj | kFInterp;
         } else {
           st |= kStTree;
@@ -381,17 +373,24 @@ __device__ __forceinline__ void level_tile(const BatchArgs &Bt, const LevelArgs 
         }
       } else {
         const int k0 = (int)(kind - kKeyGhost0);
-        ob = 8 * (int)idx;
         cmk = (uint8_t)(2 + k0);
 #pragma unroll
         for (int c = 0; c < 8; c++) spm |= (uint8_t)(((raw >> c_mirror[k0][c]) & 1) << c);
       }
     }
     sKey[off + i] = key;
-    sOb[off + i] = ob;
     sSf[off + i] = sf;
     sSpm[off + i] = spm;
     sCmk[off + i] = cmk;
+  };
+  // a present slot's place in its source: the oct's first cell, or the injected cell (of
+  // the coarser level, or where the plan and the launch do not match, which is reported
+  // and reads cell 0)
+  auto source_of = [&](uint32_t key, uint8_t sf, int cmk) -> long long {
+    const uint32_t kind = key >> 28, idx = key & 0x0FFFFFFFu;
+    if (cmk != 1) return 8LL * idx;
+    if (!(sf & kFInj)) return 0;
+    return kind == kKeyInj ? (long long)idx : (long long)__ldg(A.vcell + 7 * (size_t)idx);
   };
   auto split_of = [&](uint32_t key) -> uint8_t {
     const uint32_t kind = key >> 28;
@@ -433,11 +432,12 @@ __device__ __forceinline__ void level_tile(const BatchArgs &Bt, const LevelArgs 
         continue;
       }
       const int cmk = sCmk[sg];
+      const long long ob = source_of(sKey[sg], sf, cmk);
       double x0[5], x1[5];
       double t0[NTR > 0 ? NTR : 1] = {}, t1[NTR > 0 ? NTR : 1] = {};  // tracers of the two cells
       if (cmk == 1) {  // injected coarser cell: one value for both children
         const bool inj = sf & kFInj;
-        const double *p = (inj ? Wc : W) + (long long)sOb[sg];
+        const double *p = (inj ? Wc : W) + ob;
         const long long stride = inj ? nc8 : N8;
 #pragma unroll
         for (int v = 0; v < 5; v++) x0[v] = x1[v] = ld_state<COH>(p + v * stride);
@@ -446,7 +446,7 @@ __device__ __forceinline__ void level_tile(const BatchArgs &Bt, const LevelArgs 
           const long long ts = inj ? nc8 : N8;
           if (px != nullptr) {
 #pragma unroll
-            for (int t = 0; t < NTR; t++) t0[t] = t1[t] = ld_state<COH>(px + t * ts + (long long)sOb[sg]);
+            for (int t = 0; t < NTR; t++) t0[t] = t1[t] = ld_state<COH>(px + t * ts + ob);
           } else {
             st |= kStTree;
           }
@@ -455,7 +455,7 @@ __device__ __forceinline__ void level_tile(const BatchArgs &Bt, const LevelArgs 
         unsigned code = (unsigned)q | (1u << 3);  // pair q, elements 0 and 1
         if (cmk >= 2) code = (mir >> (4 * (cmk - 2))) & 15u;
         const bool itp = sf & kFInterp;
-        const double *p = (itp ? A.Wv : W) + (long long)sOb[sg] + 2 * (code & 3);
+        const double *p = (itp ? A.Wv : W) + ob + 2 * (code & 3);
         const long long stride = itp ? 8 * A.nv : N8;
         const bool e0 = (code >> 2) & 1, e1 = (code >> 3) & 1;
 #pragma unroll
@@ -469,7 +469,7 @@ __device__ __forceinline__ void level_tile(const BatchArgs &Bt, const LevelArgs 
 #pragma unroll
             for (int t = 0; t < NTR; t++) {
               const double2 x =
-                  ld_state<COH>(reinterpret_cast<const double2 *>(Xs + t * N8 + (long long)sOb[sg] + 2 * (code & 3)));
+                  ld_state<COH>(reinterpret_cast<const double2 *>(Xs + t * N8 + ob + 2 * (code & 3)));
               t0[t] = e0 ? x.y : x.x;
               t1[t] = e1 ? x.y : x.x;
             }
@@ -506,7 +506,7 @@ __device__ __forceinline__ void level_tile(const BatchArgs &Bt, const LevelArgs 
           const bool all = A.azall != nullptr && ld_state<COH>(A.azall) != 0;
           unsigned code = (unsigned)q | (1u << 3);
           if (cmk >= 2) code = (mir >> (4 * (cmk - 2))) & 15u;
-          const long long ib = (long long)sOb[sg] + 2 * (code & 3);
+          const long long ib = ob + 2 * (code & 3);
           const bool a0 = all || (A.az != nullptr && A.az[ib + ((code >> 2) & 1)]);
           const bool a1 = all || (A.az != nullptr && A.az[ib + ((code >> 3) & 1)]);
           if ((f0 & kFSplit) && a0) f0 |= kFAzero;
@@ -621,13 +621,11 @@ __device__ __forceinline__ void level_tile(const BatchArgs &Bt, const LevelArgs 
       for (int v = 0; v < 5; v++) Dax[v] = (ax == 0) ? D[0][v] : ((ax == 1) ? D[1][v] : D[2][v]);
       if constexpr (F64) {
         M::face_ax(q0, Dax, Wt, k, W, st, grav ? gk : nullptr);
-        V::st(sHS, r, NRING, W[0], W[1], W[2], W[3]);
-        sHS[4 * NRING + r] = W[4];
       } else {
-        M::face_px(X, Dax, k, W, st);
-        V::st(sHS, r, NRING, W[0], W[1], W[2], W[3]);
-        V::st(sHS, NRING + r, NRING, W[4], W[5], W[6], (R)0);
+        M::face_px5(X, Dax, k, W, st);
       }
+      V::st(sHS, r, NRING, W[0], W[1], W[2], W[3]);
+      sHS[4 * NRING + r] = W[4];
     }
   }
   tile_sync<COH>();
@@ -665,17 +663,12 @@ __device__ __forceinline__ void level_tile(const BatchArgs &Bt, const LevelArgs 
         M::face_ax(q0, Dax, X, k, W, st);
       }
     } else {
-      M::face_px(X, Dax, k, W, st);
+      M::face_px5(X, Dax, k, W, st);
     }
   };
   auto ring_face = [&](int r, R W[7]) {
     V::ld(sHS, r, NRING, W[0], W[1], W[2], W[3]);
-    if constexpr (F64) {
-      W[4] = sHS[4 * NRING + r];  // 1/d and a: solve_face, ring and brick lanes together
-    } else {
-      R pad;
-      V::ld(sHS, NRING + r, NRING, W[4], W[5], W[6], pad);
-    }
+    W[4] = sHS[4 * NRING + r];  // 1/d and a: solve_face, ring and brick lanes together
   };
 
   // One face e normal to axis d between left (brick cell tL at box cell bL, or
@@ -690,10 +683,8 @@ __device__ __forceinline__ void level_tile(const BatchArgs &Bt, const LevelArgs 
       else brick_face(tL, bL, 2 * d + 1, WL);
       if (jR >= 0) ring_face(jR, WR);
       else brick_face(tR, bR, 2 * d, WR);
-      if constexpr (F64) {
-        M::face_finish(WL);
-        M::face_finish(WR);
-      }
+      M::face_finish(WL);
+      M::face_finish(WR);
       if constexpr (TRACER) {
         R xs[2 * NTR];
 #pragma unroll
@@ -1260,17 +1251,16 @@ constexpr size_t level_smem_bytes(unsigned shapes) {
 // still have to finish that level.  SHAPES: the brick shapes the levels of the
 // launch use (bit i: kShapes[i]); each level's plan names its own.
 // Occupancy targets: the FP32 kernel with 4x4x2 bricks only fits 4 CTAs per SM
-// (64 registers, 55 KB of shared memory); with 2x2x2 bricks shared memory
-// allows 2; the FP64 kernel 2 with 4x4x2 bricks (128 registers, 110 KB; its
+// (64 registers, 53 KB of shared memory), with 2x2x2 bricks 3 (80 registers, 75 KB); the FP64 kernel 2 with 4x4x2 bricks (128 registers, 110 KB; its
 // dual-energy and single-tracer variants too, through their two-round layout), 1
 // with 2x2x2 bricks.
 template <class M, unsigned SHAPES, bool DUAL = false, int NTR = 0>
 constexpr int kMinBlocks = (sizeof(typename M::R) == 8) ? ((SHAPES == 1u && NTR <= 1) ? 2 : 1)
                                                          : (SHAPES == 1u ? (NTR == 3 ? 2 : ((DUAL || NTR > 0) ? 3 : 4))
-                                                                         : (NTR == 3 ? 1 : 2));
+                                                                         : (NTR == 3 ? 1 : ((DUAL || NTR > 0) ? 2 : 3)));
 // 228 KB of shared memory per SM, 1 KB reserved per CTA
 static_assert(4 * (TileSmem<MathF32, GeomA>::bytes + 1024) <= 228 * 1024, "4 FP32 4x4x2 CTAs per SM");
-static_assert(2 * (TileSmem<MathF32, GeomB>::bytes + 1024) <= 228 * 1024, "2 FP32 2x2x2 CTAs per SM");
+static_assert(3 * (TileSmem<MathF32, GeomB>::bytes + 1024) <= 228 * 1024, "3 FP32 2x2x2 CTAs per SM");
 static_assert(2 * (TileSmem<MathF64, GeomA>::bytes + 1024) <= 228 * 1024, "2 FP64 4x4x2 CTAs per SM");
 static_assert(2 * (TileSmem<MathF64, GeomA, true>::bytes + 1024) <= 228 * 1024, "2 dual-energy FP64 4x4x2 CTAs");
 static_assert(2 * (TileSmem<MathF64, GeomA, false, 1>::bytes + 1024) <= 228 * 1024, "2 tracer FP64 4x4x2 CTAs");

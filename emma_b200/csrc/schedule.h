@@ -51,6 +51,7 @@ struct StepArgs {
   unsigned *status;
   long long wait_limit;  // bounded spin of a CTA waiting for the next job
   int lfine;             // finest level with octs
+  unsigned shapes;       // brick shapes of the tree's levels (bit i: kShapes[i])
   struct StepJobRecord *jobt;  // optional: kStepJobLog records of the jobs' releases
 };
 // One released job of a fused coarse step: the device times (ns, %globaltimer) at
