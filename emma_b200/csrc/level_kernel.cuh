@@ -1250,10 +1250,11 @@ constexpr size_t level_smem_bytes(unsigned shapes) {
 // tile waiting for a finer level (listed first) never blocks the CTAs that
 // still have to finish that level.  SHAPES: the brick shapes the levels of the
 // launch use (bit i: kShapes[i]); each level's plan names its own.
-// Occupancy targets: the FP32 kernel with 4x4x2 bricks only fits 4 CTAs per SM
-// (64 registers, 53 KB of shared memory), with 2x2x2 bricks 3 (80 registers, 75 KB); the FP64 kernel 2 with 4x4x2 bricks (128 registers, 110 KB; its
-// dual-energy and single-tracer variants too, through their two-round layout), 1
-// with 2x2x2 bricks.
+// Occupancy targets: the FP32 kernel with 4x4x2 bricks only fits 4 CTAs per SM (64
+// registers, 53 KB of shared memory), with 2x2x2 bricks 3 (80 registers, 75 KB; two at
+// 82 KB cost the cosmology tree's level 8 1.50 ms a launch instead of 1.40); the FP64
+// kernel 2 with 4x4x2 bricks (128 registers, 110 KB; its dual-energy and single-tracer
+// variants too, through their two-round layout), 1 with 2x2x2 bricks.
 template <class M, unsigned SHAPES, bool DUAL = false, int NTR = 0>
 constexpr int kMinBlocks = (sizeof(typename M::R) == 8) ? ((SHAPES == 1u && NTR <= 1) ? 2 : 1)
                                                          : (SHAPES == 1u ? (NTR == 3 ? 2 : ((DUAL || NTR > 0) ? 3 : 4))
