@@ -49,35 +49,37 @@ struct MathF64 {
   // q' = q + (a - b q) y (P. Markstein, IBM J. Res. Dev. 34 (1990) 111).  The correction
   // rounds to the IEEE quotient for a correctly rounded y; for a y one ulp off
   // (div_yy) it may miss by an ulp where a/b lies within about 2^-105 of a
-  // rounding boundary.  3 FP64 instructions instead of a division's 8 to 9 and
-  // its range check, which made the divisions more than half of the FP64
-  // instructions of a face.  Where the quotient or the remainder leaves the
-  // normal range (b 0, infinite, below 1e-290; a infinite) the result may be
-  // infinite or a NaN instead of the quotient: the callers divide again when their
-  // result is not finite.
+  // rounding boundary.  Where the quotient or the remainder leaves the normal range (b 0,
+  // infinite, below 1e-290; a infinite) the result may be infinite or a NaN instead of
+  // the quotient.
   static __device__ __forceinline__ double div_y(double a, double b, double y) {
     const double q = a * y;
     return __fma_rn(__fma_rn(-b, q, a), y, q);
   }
-  // 1 / b and sqrt(x) rounded to nearest for arguments and results in the normal range
-  // (a NaN where they are not, an ulp off where the exact value lies within about
-  // 2^-100 of a rounding boundary): a 20-bit seed (PTX rcp.approx / rsqrt.approx),
-  // one step of the binomial series, and Markstein's correction from the exact
-  // residual.  As many FP64 instructions as the IEEE operators, without their range
-  // checks and branches, three a division, which are every fourth instruction of a face.
+  // 1 / b, b and 1 / b normal: two steps of Newton's iteration y <- y + y (1 - b y)
+  // (M. J. Flynn, IEEE Trans. Comput. C-19 (1970) 702) from the 20 bits of PTX
+  // rcp.approx.  Each squares the relative error; what the second leaves, 2^-80, moves
+  // only the rounding of all-ones mantissas, whose reciprocals lie 2^-106 from a boundary
+  // (tests/fp64_math_check.cu: none of 5.8e8 others).
   static __device__ __forceinline__ double rcp(double b) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-    const double e = __fma_rn(-b, y, 1.);
-    y = __fma_rn(y, __fma_rn(e, e, e), y);
+    y = __fma_rn(y, __fma_rn(-b, y, 1.), y);
     return __fma_rn(y, __fma_rn(-b, y, 1.), y);
   }
+  // sqrt(x), x normal: Goldschmidt's coupled iteration for g -> sqrt(x) and
+  // h -> 1 / (2 sqrt(x)), then the correction by the residual x - g g (P. Markstein, Software
+  // division and square root using Goldschmidt's algorithms, Proc. 6th Conf. Real
+  // Numbers and Computers (2004) 146), from the 20 bits of PTX rsqrt.approx.  One step
+  // gives 39 bits, the correction 2^-78 before its rounding.
   static __device__ __forceinline__ double root2(double x) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double t = x * y, e = __fma_rn(-t, y, 1.);
-    const double g = __fma_rn(t, e * __fma_rn(e, 0.375, 0.5), t);
-    return __fma_rn(__fma_rn(-g, g, x), 0.5 * y, g);
+    double g = x * y, h = 0.5 * y;
+    const double r = __fma_rn(-g, h, 0.5);
+    g = __fma_rn(g, r, g);
+    h = __fma_rn(h, r, h);
+    return __fma_rn(__fma_rn(-g, g, x), h, g);
   }
   static __device__ __forceinline__ double quot(double a, double b) { return div_y(a, b, rcp(b)); }
 
@@ -90,10 +92,9 @@ struct MathF64 {
   static __device__ __forceinline__ double over_g1(double p) { return div_y(p, kGam - 1., 1. / (kGam - 1.)); }
 
   // minmod_W, beta = 1 (src/hydro_utils.c:201): 0 if the signs differ, else the
-  // smaller magnitude.  One FP64 compare and selects on the sign bits instead of
-  // the reference's nested minima and maxima, each of which costs an FP64
-  // compare, two selects and a NaN check (15 limits a cell); equal for every pair
-  // of numbers but for the sign of a zero.
+  // smaller magnitude.  One compare and selects on the sign bits instead of the
+  // reference's nested minima and maxima (15 limits a cell); equal for every pair of
+  // numbers but for the sign of a zero.
   static __device__ __forceinline__ double limit(double m, double p) {
     const double s = (fabs(m) < fabs(p)) ? m : p;
     return ((__double2hiint(m) ^ __double2hiint(p)) < 0) ? 0. : s;
@@ -207,8 +208,7 @@ struct MathF64 {
   // estimate w of x^(-1/5) good to 2^-20, one step of the series of (1 - h)^(-1/5) =
   // 1 + h/5 + 3 h^2/25 + ..., h = 1 - x w^5, which leaves an error of an ulp or two,
   // y = x w^4, a Newton correction from the residual x - y^5 at twice the precision, plus
-  // y (z - 1/5) ln x; w is an ulp or two from 1/y, one Newton step rounds it.  Some 30
-  // FP64 instructions where pow() takes a hundred or more.
+  // y (z - 1/5) ln x; w is an ulp or two from 1/y, one Newton step rounds it.
   static constexpr double kZ = 1.1102230246251565e-17 * 0.6931471805599453;  // (z - 1/5) ln 2
   static __device__ __forceinline__ double root5(double x, double &iy) {
     const float xf = (float)x;
