@@ -49,14 +49,14 @@ struct MathF64 {
   // q' = q + (a - b q) y (P. Markstein, IBM J. Res. Dev. 34 (1990) 111).  The correction
   // rounds to the IEEE quotient for a correctly rounded y; for a y one ulp off
   // (div_yy) it may miss by an ulp where a/b lies within about 2^-105 of a
-  // rounding boundary.  Where the quotient or the remainder leaves the normal range (b 0,
-  // infinite, below 1e-290; a infinite) the result may be infinite or a NaN instead of
-  // the quotient.
+  // rounding boundary.  a and b finite, b and 1/b normal; elsewhere the result may be
+  // infinite or a NaN instead of the quotient: the wave speeds, the fluxes and the level
+  // kernels' updates are computed again with the operators where they are not finite.
   static __device__ __forceinline__ double div_y(double a, double b, double y) {
     const double q = a * y;
     return __fma_rn(__fma_rn(-b, q, a), y, q);
   }
-  // 1 / b, b and 1 / b normal: two steps of Newton's iteration y <- y + y (1 - b y)
+  // 1 / b, b and 1 / b normal (elsewhere a NaN): two steps of Newton's iteration y <- y + y (1 - b y)
   // (M. J. Flynn, IEEE Trans. Comput. C-19 (1970) 702) from the 20 bits of PTX
   // rcp.approx.  Each squares the relative error; what the second leaves, 2^-80, moves
   // only the rounding of all-ones mantissas, whose reciprocals lie 2^-106 from a boundary
@@ -67,7 +67,7 @@ struct MathF64 {
     y = __fma_rn(y, __fma_rn(-b, y, 1.), y);
     return __fma_rn(y, __fma_rn(-b, y, 1.), y);
   }
-  // sqrt(x), x normal: Goldschmidt's coupled iteration for g -> sqrt(x) and
+  // sqrt(x), x normal (elsewhere, and for 0, a NaN): Goldschmidt's coupled iteration for g -> sqrt(x) and
   // h -> 1 / (2 sqrt(x)), then the correction by the residual x - g g (P. Markstein, Software
   // division and square root using Goldschmidt's algorithms, Proc. 6th Conf. Real
   // Numbers and Computers (2004) 146), from the 20 bits of PTX rsqrt.approx.  One step
@@ -82,19 +82,28 @@ struct MathF64 {
     return __fma_rn(__fma_rn(-g, g, x), h, g);
   }
   static __device__ __forceinline__ double quot(double a, double b) { return div_y(a, b, rcp(b)); }
+  // these, or (IEEE) the operators
+  template <bool IEEE>
+  static __device__ __forceinline__ double div_y(double a, double b, double y) { return IEEE ? a / b : div_y(a, b, y); }
+  template <bool IEEE>
+  static __device__ __forceinline__ double quot(double a, double b) { return IEEE ? a / b : quot(a, b); }
+  template <bool IEEE>
+  static __device__ __forceinline__ double root2(double x) { return IEEE ? sqrt(x) : root2(x); }
 
   // a / RN(b b) from y = 1 / b: y y refined by one Newton step is the reciprocal
   static __device__ __forceinline__ double div_yy(double a, double b, double y) {
     const double bb = b * b, y0 = y * y;
     return div_y(a, bb, __fma_rn(y0, __fma_rn(-bb, y0, 1.), y0));
   }
-  // p / (gamma - 1) and friends: the divisor is a constant
+  // p / (gamma - 1) and friends: the divisor is a constant (a NaN for an infinite p)
   static __device__ __forceinline__ double over_g1(double p) { return div_y(p, kGam - 1., 1. / (kGam - 1.)); }
 
   // minmod_W, beta = 1 (src/hydro_utils.c:201): 0 if the signs differ, else the
   // smaller magnitude.  One compare and selects on the sign bits instead of the
   // reference's nested minima and maxima (15 limits a cell); equal for every pair of
-  // numbers but for the sign of a zero.
+  // numbers but for the sign of a zero.  Beside a NaN cell (EMMA_ST_NAN, where the
+  // reference aborts) the slope may be a NaN where the reference's drops it; telling them
+  // apart cost 1.6% of a step in integer compares, more in branches.
   static __device__ __forceinline__ double limit(double m, double p) {
     const double s = (fabs(m) < fabs(p)) ? m : p;
     return ((__double2hiint(m) ^ __double2hiint(p)) < 0) ? 0. : s;
@@ -110,8 +119,8 @@ struct MathF64 {
 #pragma unroll
       for (int k = 0; k < 5; k++) D[dir][k] = limit(q0[k] - qm[dir][k], qp[dir][k] - q0[k]);
     // stored sound speed of the cell, as U2W/scatter computes it (src/hydro_utils.c:64,3186)
-    const double id = rcp(q0[0]);
-    const double a0 = azero ? 0. : root2(div_y(kGam * q0[4], q0[0], id));
+    // (the operators: the field's densities and pressures may be 0, a face's are floored)
+    const double id = 1. / q0[0], a0 = azero ? 0. : sqrt(div_y(kGam * q0[4], q0[0], id));
     const double daa = q0[0] * a0 * a0;
     double acc[5] = {0., 0., 0., 0., 0.};
 #pragma unroll
@@ -161,8 +170,6 @@ struct MathF64 {
     return fL + fR + (R.u - L.u);
   }
   // findPressure (src/hydro_utils.c:680): rare fallback when the hybrid estimate is negative
-  // (everything by value: an address given to a call would keep the face's states and u* in
-  // local memory on the common path too)
   struct StarState { double p, u; unsigned st; };
   static __device__ __noinline__ StarState pstar_exact(S1 L, S1 R) {
     unsigned st = 0;
@@ -243,8 +250,14 @@ struct MathF64 {
   // p* < 0 as pow() with an odd integer exponent does, and the exact solver replaces
   // both).  Inlined: a call from the middle of the solver saves the live state of the face
   // in local memory (128^3 FP64 launch 0.493 ms against 0.445).
+  template <bool IEEE>
   static __device__ __forceinline__ double2 trrs(double aL, double aR, double uL, double uR, double pL, double pR) {
-    static_assert((kGam - 1.) / (2. * kGam) == 0.2 && (2. * kGam) / (kGam - 1.) == 5., "fifth roots need gamma = 5/3");
+    constexpr double z = (kGam - 1.) / (2. * kGam), iz = (2. * kGam) / (kGam - 1.);
+    static_assert(z == 0.2 && iz == 5., "fifth roots need gamma = 5/3");
+    if constexpr (IEEE) {
+      const double pstar = pow((aL + aR - (kGam - 1.) / 2. * (uR - uL)) / (aL / pow(pL, z) + aR / pow(pR, z)), iz);
+      return make_double2(pstar, uL - 2. * aL / (kGam - 1.) * (pow(pstar / pL, z) - 1.));
+    }
     double iL, iR;
     const double rL = root5(pL, iL), rR = root5(pR, iR);
     const double r = quot(aL + aR - (kGam - 1.) / 2. * (uR - uL), div_y(aL, rL, iL) + div_y(aR, rR, iR));
@@ -255,22 +268,24 @@ struct MathF64 {
   }
 
   // findPressure_Hybrid + speedestimate*_HLLC (src/hydro_utils.c:625,1264) of two states in
-  // the face's frame
-  static __device__ __forceinline__ void speeds(const double WL[7], const double WR[7], double &SL, double &SR,
-                                                double &ustar, unsigned &st) {
-    S1 L{WL[0], WL[1], WL[4], WL[6]};
-    S1 R{WR[0], WR[1], WR[4], WR[6]};
+  // the face's frame, yL and yR their 1/d.  IEEE: by the operators and pow(), with the
+  // exact solver and the status; else negative says that p* was.
+  struct Speeds { double SL, SR, ustar; unsigned st; bool negative; };
+  template <bool IEEE>
+  static __device__ __forceinline__ Speeds speeds_of(const S1 &L, const S1 &R, double yL, double yR) {
+    Speeds v;
+    v.st = 0;
     double dbar = 0.5 * (L.d + R.d), abar = 0.5 * (L.a + R.a);
     double ppvrs = 0.5 * ((L.p + R.p) + (L.u - R.u) * dbar * abar);
     double pmax = fmax(L.p, R.p), pmin = fmin(L.p, R.p);
     double pstar = ppvrs;
     // pmax / pmin < 2: the rounded quotient is below 2 exactly where pmax < 2 pmin
     if ((pmax < 2. * pmin) && ((pmin < pstar) && (pstar < pmax))) {
-      ustar = 0.5 * ((L.u + R.u) + quot(L.p - R.p, dbar * abar));
+      v.ustar = 0.5 * ((L.u + R.u) + quot<IEEE>(L.p - R.p, dbar * abar));
     } else if (pstar < pmin) {
-      const double2 r = trrs(L.a, R.a, L.u, R.u, L.p, R.p);
+      const double2 r = trrs<IEEE>(L.a, R.a, L.u, R.u, L.p, R.p);
       pstar = r.x;
-      ustar = r.y;
+      v.ustar = r.y;
     } else {
       double p0 = fmax(0., ppvrs);
       // A = 2 / ((gamma + 1) d): the reciprocal of the rounded (gamma + 1) d from 1 / d
@@ -278,29 +293,49 @@ struct MathF64 {
         const double b = (kGam + 1.) * d, y0 = y * (1. / (kGam + 1.));
         return 2. * __fma_rn(y0, __fma_rn(-b, y0, 1.), y0);
       };
-      double AL = two_over(L.d, WL[5]), AR = two_over(R.d, WR[5]);
+      double AL = IEEE ? 2. / ((kGam + 1.) * L.d) : two_over(L.d, yL);
+      double AR = IEEE ? 2. / ((kGam + 1.) * R.d) : two_over(R.d, yR);
       double BL = (kGam - 1.) / (kGam + 1.) * L.p, BR = (kGam - 1.) / (kGam + 1.) * R.p;
-      double GL = root2(quot(AL, p0 + BL)), GR = root2(quot(AR, p0 + BR));
-      pstar = quot(GL * L.p + GR * R.p - (R.u - L.u), GL + GR);
-      ustar = 0.5 * ((L.u + R.u) + (pstar - R.p) * GR - (pstar - L.p) * GL);
+      double GL = root2<IEEE>(quot<IEEE>(AL, p0 + BL)), GR = root2<IEEE>(quot<IEEE>(AR, p0 + BR));
+      pstar = quot<IEEE>(GL * L.p + GR * R.p - (R.u - L.u), GL + GR);
+      v.ustar = 0.5 * ((L.u + R.u) + (pstar - R.p) * GR - (pstar - L.p) * GL);
     }
-    if (pstar < 0) {
+    if (IEEE && pstar < 0) {
       const StarState x = pstar_exact(L, R);
       pstar = x.p;
-      ustar = x.u;
-      st |= x.st;
+      v.ustar = x.u;
+      v.st |= x.st;
     }
-    if (pstar < 0) st |= kStNegPstar;
+    if (IEEE && pstar < 0) v.st |= kStNegPstar;
     double qL = 1., qR = 1.;
-    if (!(pstar <= WL[4])) qL = root2(1. + (kGam + 1.) / (2. * kGam) * (quot(pstar, WL[4]) - 1.));
-    if (!(pstar <= WR[4])) qR = root2(1. + (kGam + 1.) / (2. * kGam) * (quot(pstar, WR[4]) - 1.));
-    SL = L.u - L.a * qL;
-    SR = R.u + R.a * qR;
-    if (SL > SR) {
-      SL = fmin(L.u - L.a, R.u - R.a);
-      SR = fmax(L.u + L.a, R.u + R.a);
+    if (!(pstar <= L.p)) qL = root2<IEEE>(1. + (kGam + 1.) / (2. * kGam) * (quot<IEEE>(pstar, L.p) - 1.));
+    if (!(pstar <= R.p)) qR = root2<IEEE>(1. + (kGam + 1.) / (2. * kGam) * (quot<IEEE>(pstar, R.p) - 1.));
+    v.SL = L.u - L.a * qL;
+    v.SR = R.u + R.a * qR;
+    if (v.SL > v.SR) {
+      v.SL = fmin(L.u - L.a, R.u - R.a);
+      v.SR = fmax(L.u + L.a, R.u + R.a);
     }
-    if (isnan(ustar)) st |= kStNan;
+    if (IEEE && isnan(v.ustar)) v.st |= kStNan;
+    v.negative = pstar < 0;
+    return v;
+  }
+  // (Arguments and result by value: an address given to a call would keep the face's states
+  // and u* in local memory on the common path too.)
+  static __device__ __noinline__ Speeds speeds_ieee(double dL, double uL, double pL, double dR, double uR, double pR) {
+    return speeds_of<true>(S1{dL, uL, pL, sqrt(kGam * pL / dL)}, S1{dR, uR, pR, sqrt(kGam * pR / dR)}, 0., 0.);
+  }
+  static __device__ __forceinline__ void speeds(const double WL[7], const double WR[7], double &SL, double &SR,
+                                                double &ustar, unsigned &st) {
+    Speeds v = speeds_of<false>(S1{WL[0], WL[1], WL[4], WL[6]}, S1{WR[0], WR[1], WR[4], WR[6]}, WL[5], WR[5]);
+    // p* < 0, or a root or quotient out of range, each of which enters one of the speeds
+    if (v.negative || !isfinite((v.SL + v.SR) + v.ustar)) {
+      v = speeds_ieee(WL[0], WL[1], WL[4], WR[0], WR[1], WR[4]);
+      st |= v.st;
+    }
+    SL = v.SL;
+    SR = v.SR;
+    ustar = v.ustar;
   }
 
   // Face state toward face k from the slope along k's axis only (the other
@@ -330,22 +365,23 @@ struct MathF64 {
   }
   // r = {d, u_n, u_t1, u_t2, p, E, |m|^2, 1/d} of a state in the face's frame
   // (E: getE, src/hydro_utils.c:29)
+  template <bool IEEE>
   static __device__ __forceinline__ void frame_state(const double W[6], bool zax, double r[8]) {
 #pragma unroll
     for (int i = 0; i < 5; i++) r[i] = W[i];
-    r[5] = over_g1(W[4]) + 0.5 * W[0] * sum_xyz(W[1] * W[1], W[2] * W[2], W[3] * W[3], zax);
+    r[5] = div_y<IEEE>(W[4], kGam - 1., 1. / (kGam - 1.)) +
+           0.5 * W[0] * sum_xyz(W[1] * W[1], W[2] * W[2], W[3] * W[3], zax);
     const double m0 = W[0] * W[1], m1 = W[0] * W[2], m2 = W[0] * W[3];
     r[6] = sum_xyz(m0 * m0, m1 * m1, m2 * m2, zax);
     r[7] = W[5];
   }
 
-  // getflux_{X,Y,Z} of W2U(W) (src/hydro_utils.c:66,916-968) in the face frame: the
-  // reference's quotients by d and d^2 from 1/d, or (IEEE) by division
+  // getflux_{X,Y,Z} of W2U(W) (src/hydro_utils.c:66,916-968) in the face frame
   template <bool IEEE>
-  static __device__ __forceinline__ void euler_quot(const double r[8], double f[5]) {
+  static __device__ __forceinline__ void euler_rot(const double r[8], double f[5]) {
     const double d = r[0], E = r[5], y = r[7];
     const double mn = d * r[1], mt1 = d * r[2], mt2 = d * r[3];
-    auto over_d = [&](double a) { return IEEE ? a / d : div_y(a, d, y); };
+    auto over_d = [&](double a) { return div_y<IEEE>(a, d, y); };
     f[0] = mn;
     f[1] = over_d(0.5 * (3. - kGam) * mn * mn) + (kGam - 1.) * E - over_d(0.5 * (kGam - 1.) * (mt1 * mt1 + mt2 * mt2));
     f[2] = over_d(mn * mt1);
@@ -353,20 +389,57 @@ struct MathF64 {
     const double c = 0.5 * (kGam - 1.) * mn;
     f[4] = over_d(kGam * mn) * E - (IEEE ? c / (d * d) : div_yy(c, d, y)) * r[6];
   }
-  struct Flux5 { double f[5]; };
-  static __device__ __noinline__ Flux5 euler_ieee(double d, double un, double t1, double t2, double E, double mm) {
-    const double r[8] = {d, un, t1, t2, 0., E, mm, 0.};
-    Flux5 x;
-    euler_quot<true>(r, x.f);
-    return x;
+
+  // The flux of tracer t, centre fraction x, from the side of state d, un (y = 1/d): the face
+  // value's du dT / d, with the star correction unless upwind (src/hydro_utils.c:1534-1539)
+  template <bool IEEE, int NT>
+  static __device__ __forceinline__ double tracer_flux(int t, double d, double un, double y, bool upwind, double S,
+                                                       double fact, double x) {
+    const double dT = (d * Tracers<NT>::frac(t)) * x;
+    const double f = div_y<IEEE>((d * un) * dT, d, y);
+    return upwind ? f : f + (div_y<IEEE>(fact * dT, d, y) - dT) * S;
   }
-  static __device__ __forceinline__ void euler_rot(const double r[8], double f[5]) {
-    euler_quot<false>(r, f);
-    if (!isfinite(f[4])) {  // a quotient may have left div_y's range (every term of f enters f[4])
-      const Flux5 x = euler_ieee(r[0], r[1], r[2], r[3], r[5], r[6]);
-#pragma unroll
-      for (int i = 0; i < 5; i++) f[i] = x.f[i];
+  // The HLLC flux of the side with state W = {d, u_n, u_t1, u_t2, p, 1/d}: its own flux
+  // (upwind), or with the star correction of the wave of speed S.  du, fx as hllc_frame's, x
+  // the side's centre fractions; returns the star density.
+  template <bool IEEE, int NT>
+  static __device__ __forceinline__ double flux_of(const double W[6], bool zax, bool upwind, double S, double ustar,
+                                                   double G[5], double *du, const double *x, double *fx) {
+    double r[8], fact = 0.;
+    frame_state<IEEE>(W, zax, r);
+    euler_rot<IEEE>(r, G);
+    const double d = r[0], un = r[1], E = r[5], y = r[7];
+    if (upwind) {
+      if (du != nullptr) {  // Us = W2U of the upwind face state
+        du[0] = div_y<IEEE>(d * un, d, y);
+        du[1] = (E - div_y<IEEE>(0.5 * r[6], d, y));
+      }
+    } else {
+      fact = quot<IEEE>(d * (S - un), S - ustar);
+      const double Es = (div_y<IEEE>(E, d, y) + (ustar - un) * (ustar + quot<IEEE>(r[4], d * (S - un))));
+      G[0] += (fact * 1. - d) * S;
+      G[1] += (fact * ustar - d * un) * S;
+      G[2] += (fact * r[2] - d * r[2]) * S;
+      G[3] += (fact * r[3] - d * r[3]) * S;
+      G[4] += (fact * Es - E) * S;
+      if (du != nullptr) {  // the star state: momenta in x,y,z order for the sum of squares
+        const double ds = fact * 1., mn = fact * ustar, m1 = fact * r[2], m2 = fact * r[3];
+        const double mm = sum_xyz(mn * mn, m1 * m1, m2 * m2, zax);
+        du[0] = mn / ds;
+        du[1] = (fact * Es - 0.5 * mm / ds);
+      }
     }
+    if (fx != nullptr)
+      for (int t = 0; t < NT; t++) fx[t] = tracer_flux<IEEE, NT>(t, d, un, y, upwind, S, fact, x[t]);
+    return fact;
+  }
+  struct SideFlux { double G[5], du[2], fact; };  // by value, as speeds_ieee
+  static __device__ __noinline__ SideFlux flux_ieee(double d, double un, double t1, double t2, double p, double S,
+                                                    double ustar, int flags) {
+    const double W[6] = {d, un, t1, t2, p, 0.};
+    SideFlux f;
+    f.fact = flux_of<true, 1>(W, flags & 1, flags & 2, S, ustar, f.G, f.du, nullptr, nullptr);
+    return f;
   }
 
   // HLLC flux across a face (src/hydro_utils.c:2055-2138) between two states in the
@@ -394,42 +467,23 @@ struct MathF64 {
     const bool left = upwind ? (SL >= 0.) : ((SL < 0.) && (ustar >= 0.));
     const bool right = upwind || ((ustar <= 0.) && (SR > 0.));
     if (left || right) {
-      double W[7], r[8];
+      double W[6], x[NT];
 #pragma unroll
       for (int i = 0; i < 6; i++) W[i] = left ? WL[i] : WR[i];
-      frame_state(W, zax, r);
-      euler_rot(r, G);
-      const double d = r[0], un = r[1], E = r[5], y = r[7];
-      if (upwind) {
-        if (du != nullptr) {  // Us = W2U of the upwind face state
-          du[0] = div_y(d * un, d, y);
-          du[1] = (E - div_y(0.5 * r[6], d, y));
+      if (fx != nullptr)
+        for (int t = 0; t < NT; t++) x[t] = xs[2 * t + (left ? 0 : 1)];
+      const double S = left ? SL : SR;
+      flux_of<false, NT>(W, zax, upwind, S, ustar, G, du, x, fx);
+      if (!isfinite(G[4])) {  // a quotient out of range: every one enters G[4]
+        const SideFlux f = flux_ieee(W[0], W[1], W[2], W[3], W[4], S, ustar, (zax ? 1 : 0) | (upwind ? 2 : 0));
+#pragma unroll
+        for (int i = 0; i < 5; i++) G[i] = f.G[i];
+        if (du != nullptr) {
+          du[0] = f.du[0];
+          du[1] = f.du[1];
         }
-        if (fx != nullptr)  // tracers: face values from the centre fractions, flux du dT / d
-          for (int t = 0; t < NT; t++) {
-            const double dT = (d * Tracers<NT>::frac(t)) * xs[2 * t + (left ? 0 : 1)];
-            fx[t] = div_y((d * un) * dT, d, y);
-          }
-      } else {
-        const double S = left ? SL : SR;
-        const double fact = quot(d * (S - un), S - ustar);
-        const double Es = (div_y(E, d, y) + (ustar - un) * (ustar + quot(r[4], d * (S - un))));
-        G[0] += (fact * 1. - d) * S;
-        G[1] += (fact * ustar - d * un) * S;
-        G[2] += (fact * r[2] - d * r[2]) * S;
-        G[3] += (fact * r[3] - d * r[3]) * S;
-        G[4] += (fact * Es - E) * S;
-        if (fx != nullptr)  // tracer fluxes with the star correction (src/hydro_utils.c:1534-1539)
-          for (int t = 0; t < NT; t++) {
-            const double dT = (d * Tracers<NT>::frac(t)) * xs[2 * t + (left ? 0 : 1)];
-            fx[t] = div_y((d * un) * dT, d, y) + (div_y(fact * dT, d, y) - dT) * S;
-          }
-        if (du != nullptr) {  // the star state: momenta in x,y,z order for the sum of squares
-          const double ds = fact * 1., mn = fact * ustar, m1 = fact * r[2], m2 = fact * r[3];
-          const double mm = sum_xyz(mn * mn, m1 * m1, m2 * m2, zax);
-          du[0] = mn / ds;
-          du[1] = (fact * Es - 0.5 * mm / ds);
-        }
+        if (fx != nullptr)
+          for (int t = 0; t < NT; t++) fx[t] = tracer_flux<true, NT>(t, W[0], W[1], 0., upwind, S, f.fact, x[t]);
       }
     }
   }

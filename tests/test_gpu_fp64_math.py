@@ -1,8 +1,9 @@
 """FP64 quotients and powers of the plain path at the edges of their ranges.
 
 The plain path takes the quotients that share a divisor from one reciprocal
-(hydro_math.cuh div_y) and divides where that leaves the normal range: densities
-whose square over- or underflows.  Its two-rarefaction star state uses fifth roots
+(hydro_math.cuh div_y) and computes with the operators again where a wave speed or a
+flux is not finite: densities whose square over- or underflows, streams so fast that
+u +- a rounds to u.  Its two-rarefaction star state uses fifth roots
 (root5), from pow() outside the single-precision range of their estimate: pressures
 above 1e37.  Every scale against the FP64 oracle, per cell <= 1e-12 (both evaluate
 the same expressions; the bound is the one of the other parity tests), colliding and
@@ -65,3 +66,63 @@ def test_fp64_nan_cell_is_reported_and_contained(gpu):
     c = np.floor(clean.cell_centres(level) * n).astype(int)
     away = np.abs((c - c[100] + n // 2) % n - n // 2).sum(1) > 3
     assert np.array_equal(out[0][0][:, away], out[1][0][:, away])
+
+
+SCALES = [(1.0, 1.0, 1.0), (1e155, 1e149, 1e-3), (1e-155, 1e-4, 1e75), (1.0, 1e40, 1e20),
+          (1.0, 1.0, 1e20),    # hypersonic: u +- a rounds to u, zero divisors in the star state
+          (1.0, 1.0, 1e70),    # ... and the two-rarefaction p* = r^5 of receding streams overflows
+          (1.0, 1e-6, 1e62)]
+
+
+def one_step_on(kernel, trees, oracle_lib, levels, **variant):
+    """One coarse step on the brick (-1) or the column kernel and by the oracle: states, velocities
+    relative to |v| + c_s, pressures to p + d |v|^2, the energy that a pressure is a difference of."""
+    r = ResidentHydro(trees[0], precision=PREC_FP64, cfl=0.8, column=kernel, **variant)
+    r.coarse_step()
+    assert (r.column_tuning(levels)[0] > 0) == (kernel > 0)
+    _, _, err = oracle_lib.run(trees[1].firstoct, levels, levels, 1, 0.8, **variant)
+    assert err == 0 and r.status() == 0
+    g, o = r.state(levels), trees[1].get_fields(levels)[:5]
+    assert np.isfinite(o).all() and np.isfinite(g).all()
+    v2 = (o[1:4] ** 2).sum(0)
+    scale = [o[0]] + 3 * [np.sqrt(v2) + np.sqrt(5.0 / 3.0 * o[4] / o[0])] + [o[4] + o[0] * v2]
+    return max(float((np.abs(g[k] - o[k]) / scale[k]).max()) for k in range(5)), r
+
+
+@pytest.mark.parametrize("kernel", [-1, 4])
+@pytest.mark.parametrize("variant", ["plain", "dual", "tracer"])
+@pytest.mark.parametrize("scale", SCALES)
+def test_fp64_extreme_scales_on_each_kernel(gpu, scale, variant, kernel):
+    level = 4
+    trees = [box(level, *scale) for _ in range(2)]
+    if variant == "tracer":
+        trees = [OctTree(level, level, rh=True) for _ in range(2)]
+        for t in trees:
+            f = box(level, *scale).get_fields(level)[:5]
+            t.set_fields(level, *f)
+            t.set_tracer(level, f[0] * np.random.default_rng(11).uniform(0.0, 1.0, f.shape[1]))
+    worst, r = one_step_on(kernel, trees, oracle.Restatement(rh=variant == "tracer"), level,
+                           **({"dual": True} if variant == "dual" else {}))
+    assert worst <= 1e-12
+    if variant == "tracer":
+        r.download()
+        x, o = (t.get_tracer(level) for t in trees)
+        # at 1e155 the tracer flux (d u) dT / d overflows in the reference's order too
+        assert np.array_equal(np.isnan(x), np.isnan(o)) and (np.isfinite(o).all() or scale[0] == 1e155)
+        ok = ~np.isnan(o)
+        assert (np.abs(x - o)[ok] <= 1e-12 * trees[1].get_fields(level)[0][ok]).all()
+
+
+@pytest.mark.parametrize("kernel", [-1, 4])
+@pytest.mark.parametrize("dual", [False, True])
+@pytest.mark.parametrize("where", ["cell", "half"])
+def test_fp64_cells_without_pressure(gpu, where, dual, kernel):
+    """p = 0 cells (cold gas): a sound speed of 0 in the predictor, the floor on their faces."""
+    level = 4
+    trees = [box(level, 1.0, 1.0, 1.0) for _ in range(2)]
+    for t in trees:
+        f = t.get_fields(level)[:5]
+        cold = t.cell_centres(level)[:, 0] < 0.5 if where == "half" else np.arange(f.shape[1]) == 100
+        f[4, cold] = 0.0
+        t.set_fields(level, *f)
+    assert one_step_on(kernel, trees, oracle.Restatement(), level, **({"dual": True} if dual else {}))[0] <= 1e-12
