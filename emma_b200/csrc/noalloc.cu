@@ -8,15 +8,16 @@
 // caller passes the level state already on the device and receives dt; the
 // reduction's scratch is a fixed array inside this library.
 //
-// Scratch: g_dt_scratch, a file-scope __device__ array of kMaxBlocks + 1 + kCounters
-// 64-bit slots (128.5 KiB) that every GPU which loads the library holds until the
-// process exits.  Slot b < kMaxBlocks receives the maximum signal speed of block b, slot
-// kMaxBlocks the maximum over the blocks; every one of these that a call reads is
-// written earlier in the same call.  The others count a call's finished blocks: call k
-// takes counter k mod kCounters and clears that of call k + kCounters / 2, so a counter
-// starts at zero whatever became of the call that used it before.  Calls whose kernels
-// overlap on the GPU (different streams, or several host threads) share the array and
-// race: serialise them on one stream.
+// Scratch: g_dt_scratch, a file-scope __device__ array of kMaxBlocks + 2 64-bit slots
+// (128 KiB + 16 B) that every GPU which loads the library holds until the process exits.
+// Slot b < kMaxBlocks receives the maximum signal speed of block b, slot kMaxBlocks the
+// maximum over the blocks; every one of these that a call reads is written earlier in the
+// same call.  The last slot counts a call's finished blocks, above the call's own
+// number: calls are numbered from 1, a block first raises the slot to its call's number
+// with no block counted, so it counts from zero whatever any call before it left there, one
+// that never ran, failed or overlapped another.  Calls whose kernels overlap on the GPU
+// (different streams, or several host threads) share the array and race: serialise them
+// on one stream.
 //
 // Host code only ever uses the array's device address, obtained once per device
 // with cudaGetSymbolAddress on the first call made while that device is
@@ -40,14 +41,16 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kMaxBlocks = 16384;
-constexpr int kCounters = 64;
+constexpr int kCountBits = 20;  // of the counting slot; the call's number above them
 constexpr long long kMaxCells = 2048LL * kMaxBlocks;  // 33,554,432 cells (a 256^3 level is 16,777,216)
 constexpr int kMaxDevices = 64;
+static_assert(kMaxBlocks < (1 << kCountBits), "the blocks of a call in the counting slot's low bits");
 
-static __device__ __align__(256) unsigned long long g_dt_scratch[kMaxBlocks + 1 + kCounters];
+static __device__ __align__(256) unsigned long long g_dt_scratch[kMaxBlocks + 2];
 
 std::atomic<unsigned long long *> g_scratch_addr[kMaxDevices];  // zero-initialised (static storage)
-std::atomic<unsigned> g_calls[kMaxDevices];
+std::atomic<unsigned long long> g_calls[kMaxDevices];
+std::atomic<int> g_sms[kMaxDevices];
 
 __device__ __forceinline__ double block_max(double m) {
   __shared__ double part[kThreads / 32];
@@ -67,7 +70,9 @@ __device__ __forceinline__ double block_max(double m) {
 // read-back).  Small levels take one cell a thread (latency; 128^3 32.9 -> 29.8 us), large
 // ones eight at a time (256^3 130 -> 127 us, 5.3 TB/s with the call's fixed cost).
 __global__ void __launch_bounds__(kThreads) dt_kernel(const double *__restrict__ W, long long n8, int per_thread,
-                                                      unsigned call, unsigned long long *scratch) {
+                                                      unsigned long long call, unsigned long long *scratch) {
+  unsigned long long *count = scratch + kMaxBlocks + 1;
+  if (threadIdx.x == 0) atomicMax(count, call << kCountBits);  // here, beside the loads
   double m = 0.;
   const long long base = (long long)blockIdx.x * kThreads * per_thread + threadIdx.x;
   auto cell = [&](long long i) {
@@ -88,10 +93,8 @@ __global__ void __launch_bounds__(kThreads) dt_kernel(const double *__restrict__
   __shared__ bool last;
   if (threadIdx.x == 0) {
     scratch[blockIdx.x] = (unsigned long long)__double_as_longlong(m);
-    unsigned long long *count = scratch + kMaxBlocks + 1;
-    if (blockIdx.x == 0) count[(call + kCounters / 2) % kCounters] = 0ULL;
     __threadfence();
-    last = atomicAdd(count + call % kCounters, 1ULL) == gridDim.x - 1;
+    last = atomicAdd(count, 1ULL) == (call << kCountBits) + gridDim.x - 1;
   }
   __syncthreads();  // also: block_max's shared memory is free again
   if (!last) return;
@@ -122,23 +125,29 @@ extern "C" int emma_hydro_level_dt_noalloc(const double *d_state, long long ncel
     void *p = nullptr;
     if (cudaGetSymbolAddress(&p, g_dt_scratch) != cudaSuccess || p == nullptr) return EMMA_ST_CUDA;
     scratch = static_cast<unsigned long long *>(p);
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return EMMA_ST_CUDA;
+    g_sms[dev].store(sms, std::memory_order_relaxed);
     g_scratch_addr[dev].store(scratch, std::memory_order_release);
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   double smax = 0.;
   if (ncells > 0) {
-    // enough cells a thread to keep to 8 blocks an SM (148), a power of two up to 8; beyond
-    // 4096 blocks 16, or the counting of the blocks shows
+    // enough cells a thread to keep to 8 blocks an SM, a power of two up to 8; beyond 4096
+    // blocks 16, or the counting of the blocks shows
+    const long long resident = 8LL * kThreads * g_sms[dev].load(std::memory_order_relaxed);
     int per = 1;
-    while (per < 8 && ncells > (long long)kThreads * per * 8 * 148) per *= 2;
+    while (per < 8 && ncells > resident * per) per *= 2;
     if (ncells > (long long)kThreads * per * 4096) per = 16;
     const int nblocks = (int)((ncells + (long long)kThreads * per - 1) / ((long long)kThreads * per));
-    dt_kernel<<<nblocks, kThreads, 0, s>>>(d_state, ncells, per, g_calls[dev].fetch_add(1u), scratch);
+    dt_kernel<<<nblocks, kThreads, 0, s>>>(d_state, ncells, per, g_calls[dev].fetch_add(1u) + 1u, scratch);
     if (cudaGetLastError() != cudaSuccess) return EMMA_ST_CUDA;
     unsigned long long bits = 0;
     if (cudaMemcpyAsync(&bits, scratch + kMaxBlocks, sizeof(bits), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-        cudaStreamSynchronize(s) != cudaSuccess)
+        cudaStreamSynchronize(s) != cudaSuccess) {
+      cudaGetLastError();  // a call refused here (a stream under capture) is not the next call's error
       return EMMA_ST_CUDA;
+    }
     std::memcpy(&smax, &bits, sizeof(smax));
   }
   // L_comptstep_hydro's final step (src/advanceamr.c:135)

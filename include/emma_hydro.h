@@ -343,7 +343,7 @@ int emma_hydro_plan_stats(struct OCT **firstoct, int lcoarse, int lmax, int tran
  * `ncells` doubles); *dt_out receives what emma_hydro_comptstep returns for
  * that state at `level` with Courant number `cfl`.  Works on the current
  * device and needs neither emma_hydro_init nor a resident tree.
- * Scratch is a fixed 128.5 KiB array inside the library, held on every GPU that
+ * Scratch is a fixed 128 KiB array inside the library, held on every GPU that
  * loads it until exit, so ncells is limited to 33554432 (EMMA_ST_ARG beyond).
  * The first call on each device looks up the array's address (make it before
  * any stream capture).  Calls overlapping on the GPU share the array and race.

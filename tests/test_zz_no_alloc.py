@@ -71,6 +71,40 @@ def test_noalloc_dt_limits(gpu):
     assert code == 0 and dt == 1e9
 
 
+@pytest.mark.gpu
+def test_noalloc_dt_after_refused_calls(gpu):
+    """A call on a stream under capture is refused (its kernel never runs, the library's calls
+    are counted on): every later one still returns its own state's dt, over more calls than
+    any ring of counters holds, with more and fewer blocks than the call before."""
+    import torch
+    driver = ctypes.CDLL("libcuda.so.1")
+    s = torch.cuda.Stream()
+    stream = ctypes.c_void_p(s.cuda_stream)
+    rng = np.random.default_rng(5)
+    states, expected = [], []
+    for n in (256, 5000, 700, 300000):
+        d, p = (np.exp(rng.uniform(-1, 1, n)) for _ in range(2))
+        w = np.stack([d, *(rng.uniform(-1, 1, n) for _ in range(3)), p])
+        states.append(torch.from_numpy(w).cuda())
+        # as L_comptstep_hydro rounds it, numpy's operators being IEEE's
+        speed = np.sqrt(w[1] * w[1] + w[2] * w[2] + w[3] * w[3]) + np.sqrt((5.0 / 3.0) * w[4] / w[0])
+        expected.append(0.5 ** 5 * CFL / (speed.max() * 3.0))
+    torch.cuda.synchronize()
+    refused = 0
+    for call in range(300):
+        i = int(rng.integers(4))
+        if call in (7, 60, 61, 150):
+            graph = ctypes.c_void_p()
+            assert driver.cuStreamBeginCapture_v2(stream, 1) == 0  # this thread only
+            code, _ = noalloc_dt(states[i].data_ptr(), states[i].shape[1], 5, stream)
+            driver.cuStreamEndCapture(stream, ctypes.byref(graph))
+            assert code != 0 and not graph.value
+            refused += 1
+        code, dt = noalloc_dt(states[i].data_ptr(), states[i].shape[1], 5, stream)
+        assert (code, dt) == (0, expected[i]), (call, refused)
+    assert refused == 4
+
+
 def test_noalloc_rejects_arguments_on_host():
     """Rejections happen before any CUDA call (no GPU needed)."""
     fake = ctypes.c_void_p(256)  # never dereferenced: every case below is refused first
