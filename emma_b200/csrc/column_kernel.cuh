@@ -131,12 +131,15 @@ using Col32 = Col<float, column_height(false), DUAL, NTR>;
 
 // The warp's maximum of the next CFL step's |v| + c_s (src/advanceamr.c:122-128) after
 // each of its threads wrote the state Wout: exact in FP64 for every cell that may raise
-// wmax (warp-uniform); an FP32 estimate (relative error below 2e-6 where it has not
-// underflowed) screens the others out, whole warps at a time.
+// wmax (warp-uniform); an FP32 estimate (relative error below 2e-6) screens the others
+// out, whole warps at a time.  The cell is looked at where the estimate does not hold: it
+// underflowed (below 1e-15), the quotient is 0 (densities beyond FP32, or beyond the 2^126
+// from which the approximate division gives 0), the density is below FP32's normal numbers
+// (c_s > 1e13 then, with pressures >= 1e-10), or it is no number.
 __device__ __forceinline__ double column_cfl_max(const double Wout[5], double wmax) {
-  const float u = (float)Wout[1], v = (float)Wout[2], w = (float)Wout[3];
-  const float s32 = sqrtf(u * u + v * v + w * w) + sqrtf(5.f / 3.f * (float)Wout[4] / (float)Wout[0]);
-  const bool cand = !(s32 < (float)wmax * (1.f - 1e-5f)) || s32 < 1e-15f;
+  const float u = (float)Wout[1], v = (float)Wout[2], w = (float)Wout[3], q = (float)Wout[4] / (float)Wout[0];
+  const float s32 = sqrtf(u * u + v * v + w * w) + sqrtf(5.f / 3.f * q);
+  const bool cand = !(s32 < (float)wmax * (1.f - 1e-5f)) || !(s32 > 1e-15f && s32 < 1e13f) || !(q > 0.f);
   if (__any_sync(0xffffffffu, cand)) {
     double ex = 0.;
     if (cand) {

@@ -126,3 +126,21 @@ def test_fp64_cells_without_pressure(gpu, where, dual, kernel):
         f[4, cold] = 0.0
         t.set_fields(level, *f)
     assert one_step_on(kernel, trees, oracle.Restatement(), level, **({"dual": True} if dual else {}))[0] <= 1e-12
+
+
+@pytest.mark.parametrize("scale", [(1e45, 1e30, 1e-9), (1e38, 1e23, 1e-9), (1e-43, 1e-10, 1.0), (1e30, 1e40, 1e-3)])
+def test_fp64_time_steps_outside_single_precision(gpu, scale):
+    """From the second step on dt comes from the maximum that the level kernel leaves; the
+    column kernel screens cells by an FP32 estimate, which these densities or pressures
+    leave: the bricks' maximum, bit for bit, and the oracle's time."""
+    level, steps, out = 5, 4, []
+    for kernel in (-1, 2, 32):
+        r = ResidentHydro(box(level, *scale), precision=PREC_FP64, cfl=0.8, column=kernel)
+        for _ in range(steps):
+            r.coarse_step()
+        assert r.status() == 0
+        out.append((r.tsim, r.state(level)))
+    assert all(t == out[0][0] and np.array_equal(s, out[0][1]) for t, s in out[1:])
+    to = box(level, *scale)
+    t, _, err = oracle.Restatement().run(to.firstoct, level, level, steps, 0.8)
+    assert err == 0 and abs(out[0][0] - t) <= 1e-12 * t
