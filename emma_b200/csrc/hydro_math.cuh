@@ -119,8 +119,8 @@ struct MathF64 {
 #pragma unroll
       for (int k = 0; k < 5; k++) D[dir][k] = limit(q0[k] - qm[dir][k], qp[dir][k] - q0[k]);
     // stored sound speed of the cell, as U2W/scatter computes it (src/hydro_utils.c:64,3186)
-    // (the operators: the field's densities and pressures may be 0, a face's are floored)
-    const double id = 1. / q0[0], a0 = azero ? 0. : sqrt(div_y(kGam * q0[4], q0[0], id));
+    // (sqrt, not root2: the field's pressures may be 0, a face's are floored)
+    const double id = rcp(q0[0]), a0 = azero ? 0. : sqrt(div_y(kGam * q0[4], q0[0], id));
     const double daa = q0[0] * a0 * a0;
     double acc[5] = {0., 0., 0., 0., 0.};
 #pragma unroll
@@ -269,8 +269,10 @@ struct MathF64 {
 
   // findPressure_Hybrid + speedestimate*_HLLC (src/hydro_utils.c:625,1264) of two states in
   // the face's frame, yL and yR their 1/d.  IEEE: by the operators and pow(), with the
-  // exact solver and the status; else negative says that p* was.
-  struct Speeds { double SL, SR, ustar; unsigned st; bool negative; };
+  // exact solver and the status; else `again` says that this is needed: p* is negative, or
+  // one of the speeds a NaN, as a root or quotient out of range makes them (never an
+  // infinity that the operators don't give).
+  struct Speeds { double SL, SR, ustar; unsigned st; bool again; };
   template <bool IEEE>
   static __device__ __forceinline__ Speeds speeds_of(const S1 &L, const S1 &R, double yL, double yR) {
     Speeds v;
@@ -307,17 +309,21 @@ struct MathF64 {
       v.st |= x.st;
     }
     if (IEEE && pstar < 0) v.st |= kStNegPstar;
+    v.again = pstar < 0;
     double qL = 1., qR = 1.;
     if (!(pstar <= L.p)) qL = root2<IEEE>(1. + (kGam + 1.) / (2. * kGam) * (quot<IEEE>(pstar, L.p) - 1.));
     if (!(pstar <= R.p)) qR = root2<IEEE>(1. + (kGam + 1.) / (2. * kGam) * (quot<IEEE>(pstar, R.p) - 1.));
     v.SL = L.u - L.a * qL;
     v.SR = R.u + R.a * qR;
-    if (v.SL > v.SR) {
-      v.SL = fmin(L.u - L.a, R.u - R.a);
-      v.SR = fmax(L.u + L.a, R.u + R.a);
+    if (!(v.SL <= v.SR)) {
+      if (v.SL > v.SR) {
+        v.SL = fmin(L.u - L.a, R.u - R.a);
+        v.SR = fmax(L.u + L.a, R.u + R.a);
+      } else {
+        v.again = true;
+      }
     }
     if (IEEE && isnan(v.ustar)) v.st |= kStNan;
-    v.negative = pstar < 0;
     return v;
   }
   // (Arguments and result by value: an address given to a call would keep the face's states
@@ -328,8 +334,7 @@ struct MathF64 {
   static __device__ __forceinline__ void speeds(const double WL[7], const double WR[7], double &SL, double &SR,
                                                 double &ustar, unsigned &st) {
     Speeds v = speeds_of<false>(S1{WL[0], WL[1], WL[4], WL[6]}, S1{WR[0], WR[1], WR[4], WR[6]}, WL[5], WR[5]);
-    // p* < 0, or a root or quotient out of range, each of which enters one of the speeds
-    if (v.negative || !isfinite((v.SL + v.SR) + v.ustar)) {
+    if (v.again || isnan(v.ustar)) {
       v = speeds_ieee(WL[0], WL[1], WL[4], WR[0], WR[1], WR[4]);
       st |= v.st;
     }
