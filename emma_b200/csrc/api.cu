@@ -149,7 +149,7 @@ struct Ctx {
   int *d_work_all = nullptr;     // batched work list, finest level first
   int nwork_all = 0;
   cudaGraphExec_t graph = nullptr;
-  int graph_nsub = -1, graph_prec = -1, graph_col = -2, graph_colx = -2, graph_colb = -2, graph_groups = -3;
+  int graph_nsub = -1, graph_prec = -1, graph_col = -2, graph_colx = -2, graph_colb = -2, graph_octs = -2, graph_groups = -3;
   bool graph_is_fused = false;   // the captured coarse step is one fused kernel
   int graph_kernels = 0;         // kernel nodes of the captured coarse step
   // drop-in cache: one mirror of levels L-1..L+1 per advanced level L, so that a
@@ -379,6 +379,7 @@ void drop_graph() {
   g.graph_col = -2;
   g.graph_colx = -2;
   g.graph_colb = -2;
+  g.graph_octs = -2;
   g.graph_groups = -3;
   g.graph_is_fused = false;
   g.graph_kernels = 0;
@@ -1023,7 +1024,7 @@ bool emit_coarse_step(int nsub) {
 bool ensure_graph(int nsub) {
   if (g.graph && g.graph_nsub == nsub && g.graph_prec == g.opt.precision && g.graph_col == g.opt.column &&
       g.graph_colx == g.opt.column_xshfl && g.graph_colb == g.opt.column_balanced &&
-      g.graph_groups == g.step_groups)
+      g.graph_octs == g.opt.tile_octs && g.graph_groups == g.step_groups)  // all that column_nz() and its split go by
     return true;
   drop_graph();
   cudaGraph_t graph = nullptr;
@@ -1055,6 +1056,7 @@ bool ensure_graph(int nsub) {
   g.graph_col = g.opt.column;
   g.graph_colx = g.opt.column_xshfl;
   g.graph_colb = g.opt.column_balanced;
+  g.graph_octs = g.opt.tile_octs;
   g.graph_groups = g.step_groups;
   g.graph_kernels = kn;
   return true;

@@ -62,3 +62,23 @@ def test_fp64_keeps_the_brick_kernel(gpu, kw):
     """Other transmissive faces, whose ghosts are not copies of the boundary cells on every
     side, and a forced brick shape."""
     assert run(5, PREC_FP64, "plain", steps=1, **kw)[2] == 0
+
+
+def test_captured_step_follows_a_forced_brick_shape(gpu):
+    """tile_octs set between two steps of a resident tree decides the kernel (FP64: the bricks
+    when it is forced): the captured step of the other kernel is not launched again."""
+    rng = np.random.default_rng(3)
+    t = OctTree(5, 5)
+    n = 8 * t.noct(5)
+    d, p = (np.exp(rng.uniform(-1, 1, n)) for _ in range(2))
+    t.set_fields(5, d, *(rng.uniform(-1, 1, n) for _ in range(3)), p)
+    r = ResidentHydro(t, precision=PREC_FP64, cfl=0.8, column=4)
+    launches = []
+    for octs in (0, 32, 0):
+        r.tile_octs = octs
+        r._apply()
+        r.coarse_step()
+        assert (r.column_tuning(5)[0] > 0) == (octs == 0)
+        launches.append(r.graph_info()[3])
+    # column kernel: its last CTA ends the step; bricks: CFL, begin, level, end
+    assert launches == [2, 4, 2] and r.status() == 0
