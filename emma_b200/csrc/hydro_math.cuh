@@ -269,9 +269,9 @@ struct MathF64 {
 
   // findPressure_Hybrid + speedestimate*_HLLC (src/hydro_utils.c:625,1264) of two states in
   // the face's frame, yL and yR their 1/d.  IEEE: by the operators and pow(), with the
-  // exact solver and the status; else `again` says that this is needed: p* is negative, or
-  // one of the speeds a NaN, as a root or quotient out of range makes them (never an
-  // infinity that the operators don't give).
+  // exact solver and the status; else `again` says that these are needed: p* is negative, or
+  // SL or SR a NaN, as a root or quotient out of range makes them (never an infinity that
+  // the operators don't give).
   struct Speeds { double SL, SR, ustar; unsigned st; bool again; };
   template <bool IEEE>
   static __device__ __forceinline__ Speeds speeds_of(const S1 &L, const S1 &R, double yL, double yR) {
@@ -325,22 +325,6 @@ struct MathF64 {
     }
     if (IEEE && isnan(v.ustar)) v.st |= kStNan;
     return v;
-  }
-  // (Arguments and result by value: an address given to a call would keep the face's states
-  // and u* in local memory on the common path too.)
-  static __device__ __noinline__ Speeds speeds_ieee(double dL, double uL, double pL, double dR, double uR, double pR) {
-    return speeds_of<true>(S1{dL, uL, pL, sqrt(kGam * pL / dL)}, S1{dR, uR, pR, sqrt(kGam * pR / dR)}, 0., 0.);
-  }
-  static __device__ __forceinline__ void speeds(const double WL[7], const double WR[7], double &SL, double &SR,
-                                                double &ustar, unsigned &st) {
-    Speeds v = speeds_of<false>(S1{WL[0], WL[1], WL[4], WL[6]}, S1{WR[0], WR[1], WR[4], WR[6]}, WL[5], WR[5]);
-    if (v.again || isnan(v.ustar)) {
-      v = speeds_ieee(WL[0], WL[1], WL[4], WR[0], WR[1], WR[4]);
-      st |= v.st;
-    }
-    SL = v.SL;
-    SR = v.SR;
-    ustar = v.ustar;
   }
 
   // Face state toward face k from the slope along k's axis only (the other
@@ -406,10 +390,10 @@ struct MathF64 {
   }
   // The HLLC flux of the side with state W = {d, u_n, u_t1, u_t2, p, 1/d}: its own flux
   // (upwind), or with the star correction of the wave of speed S.  du, fx as hllc_frame's, x
-  // the side's centre fractions; returns the star density.
+  // the side's centre fractions.
   template <bool IEEE, int NT>
-  static __device__ __forceinline__ double flux_of(const double W[6], bool zax, bool upwind, double S, double ustar,
-                                                   double G[5], double *du, const double *x, double *fx) {
+  static __device__ __forceinline__ void flux_of(const double W[6], bool zax, bool upwind, double S, double ustar,
+                                                 double G[5], double *du, const double *x, double *fx) {
     double r[8], fact = 0.;
     frame_state<IEEE>(W, zax, r);
     euler_rot<IEEE>(r, G);
@@ -436,15 +420,6 @@ struct MathF64 {
     }
     if (fx != nullptr)
       for (int t = 0; t < NT; t++) fx[t] = tracer_flux<IEEE, NT>(t, d, un, y, upwind, S, fact, x[t]);
-    return fact;
-  }
-  struct SideFlux { double G[5], du[2], fact; };  // by value, as speeds_ieee
-  static __device__ __noinline__ SideFlux flux_ieee(double d, double un, double t1, double t2, double p, double S,
-                                                    double ustar, int flags) {
-    const double W[6] = {d, un, t1, t2, p, 0.};
-    SideFlux f;
-    f.fact = flux_of<true, 1>(W, flags & 1, flags & 2, S, ustar, f.G, f.du, nullptr, nullptr);
-    return f;
   }
 
   // HLLC flux across a face (src/hydro_utils.c:2055-2138) between two states in the
@@ -455,12 +430,16 @@ struct MathF64 {
   // Us.E - |Us.m|^2 / (2 Us.d) (src/hydro_utils.c:2126-2128).
   // xs, fx (tracer builds, optional): the centre fractions of the NT tracers,
   // xs[2 t] left and xs[2 t + 1] right, and their fluxes fx[t].
-  template <int NT = 1>
-  static __device__ __forceinline__ void hllc_frame(const double WL[7], const double WR[7], bool zax, double G[5],
-                                                    unsigned &st, double *du = nullptr, const double *xs = nullptr,
-                                                    double *fx = nullptr) {
-    double SL, SR, ustar;
-    speeds(WL, WR, SL, SR, ustar, st);
+  //
+  // hllc_any<true>: by the operators, pow() and the exact solver, with the status.
+  // hllc_any<false>: without them; the result says whether they are needed: p* < 0, or a root
+  // or quotient out of range, each of which leaves a NaN in a wave speed or a flux that is not
+  // finite.
+  template <bool IEEE, int NT>
+  static __device__ __forceinline__ bool hllc_any(const double WL[7], const double WR[7], bool zax, double G[5],
+                                                  unsigned &st, double *du, const double *xs, double *fx) {
+    const Speeds v = speeds_of<IEEE>(S1{WL[0], WL[1], WL[4], WL[6]}, S1{WR[0], WR[1], WR[4], WR[6]}, WL[5], WR[5]);
+    if (IEEE) st |= v.st;
 #pragma unroll
     for (int i = 0; i < 5; i++) G[i] = 0.;
     if (du != nullptr) du[0] = du[1] = 0.;
@@ -468,28 +447,69 @@ struct MathF64 {
       for (int t = 0; t < NT; t++) fx[t] = 0.;
     // the upwind side's flux, plus the star correction inside the fan; no flux when
     // neither side's condition holds (a NaN speed)
-    const bool upwind = SL >= 0. || SR <= 0.;
-    const bool left = upwind ? (SL >= 0.) : ((SL < 0.) && (ustar >= 0.));
-    const bool right = upwind || ((ustar <= 0.) && (SR > 0.));
+    const bool upwind = v.SL >= 0. || v.SR <= 0.;
+    const bool left = upwind ? (v.SL >= 0.) : ((v.SL < 0.) && (v.ustar >= 0.));
+    const bool right = upwind || ((v.ustar <= 0.) && (v.SR > 0.));
     if (left || right) {
       double W[6], x[NT];
 #pragma unroll
       for (int i = 0; i < 6; i++) W[i] = left ? WL[i] : WR[i];
       if (fx != nullptr)
         for (int t = 0; t < NT; t++) x[t] = xs[2 * t + (left ? 0 : 1)];
-      const double S = left ? SL : SR;
-      flux_of<false, NT>(W, zax, upwind, S, ustar, G, du, x, fx);
-      if (!isfinite(G[4])) {  // a quotient out of range: every one enters G[4]
-        const SideFlux f = flux_ieee(W[0], W[1], W[2], W[3], W[4], S, ustar, (zax ? 1 : 0) | (upwind ? 2 : 0));
+      flux_of<IEEE, NT>(W, zax, upwind, left ? v.SL : v.SR, v.ustar, G, du, x, fx);
+    }
+    bool again = v.again || isnan(v.ustar) || !isfinite(G[4]);
+    if (fx != nullptr)
+      for (int t = 0; t < NT; t++) again = again || !isfinite(fx[t]);
+    return again;
+  }
+  // The rare faces.  Once, at the end of a face, and by value: a call in the middle of the
+  // solver, for the exact p* alone or for the wave speeds, keeps what lives across it in
+  // few registers (FP64 128^3 step 0.405 ms instead of 0.390, dual energy 0.494 instead of
+  // 0.456), an address given to one keeps it in local memory.
+  template <int NT>
+  struct FaceStates { double l[5], r[5], xs[2 * NT]; int zax; };
+  template <int NT>
+  struct FaceFlux { double G[5], du[2], fx[NT]; unsigned st; };
+  template <int NT>
+  static __device__ __noinline__ FaceFlux<NT> hllc_again(FaceStates<NT> s) {
+    FaceFlux<NT> x;
+    double WL[7], WR[7];
+    for (int i = 0; i < 5; i++) {
+      WL[i] = s.l[i];
+      WR[i] = s.r[i];
+    }
+    WL[5] = WR[5] = 0.;  // not used
+    WL[6] = sqrt(kGam * WL[4] / WL[0]);
+    WR[6] = sqrt(kGam * WR[4] / WR[0]);
+    x.st = 0;
+    hllc_any<true, NT>(WL, WR, s.zax, x.G, x.st, x.du, s.xs, x.fx);
+    return x;
+  }
+
+  template <int NT = 1>
+  static __device__ __forceinline__ void hllc_frame(const double WL[7], const double WR[7], bool zax, double G[5],
+                                                    unsigned &st, double *du = nullptr, const double *xs = nullptr,
+                                                    double *fx = nullptr) {
+    if (hllc_any<false, NT>(WL, WR, zax, G, st, du, xs, fx)) {
+      FaceStates<NT> f;
 #pragma unroll
-        for (int i = 0; i < 5; i++) G[i] = f.G[i];
-        if (du != nullptr) {
-          du[0] = f.du[0];
-          du[1] = f.du[1];
-        }
-        if (fx != nullptr)
-          for (int t = 0; t < NT; t++) fx[t] = tracer_flux<true, NT>(t, W[0], W[1], 0., upwind, S, f.fact, x[t]);
+      for (int i = 0; i < 5; i++) {
+        f.l[i] = WL[i];
+        f.r[i] = WR[i];
       }
+      for (int t = 0; t < 2 * NT; t++) f.xs[t] = xs != nullptr ? xs[t] : 0.;
+      f.zax = zax;
+      const FaceFlux<NT> x = hllc_again<NT>(f);
+#pragma unroll
+      for (int i = 0; i < 5; i++) G[i] = x.G[i];
+      if (du != nullptr) {
+        du[0] = x.du[0];
+        du[1] = x.du[1];
+      }
+      if (fx != nullptr)
+        for (int t = 0; t < NT; t++) fx[t] = x.fx[t];
+      st |= x.st;
     }
   }
 
