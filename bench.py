@@ -505,8 +505,8 @@ def main():
                          "api": "emma_hydro_set_level_state + coarse step + emma_hydro_get_level_state, pinned host"},
         "autotune": {"mixed": mixed["autotune"], "fp64": fp64["autotune"],
                      "candidates": "brick 4x4x2 octs x1 or 2x2x2 octs x4 per 256-thread tile, 1..occupancy CTAs "
-                                   "per SM; mixed path on complete periodic levels without split cells: the column "
-                                   "kernel (16x16-cell columns) with 2..64 cell planes per work item"},
+                                   "per SM; complete levels without split cells, periodic or transmissive in x: the "
+                                   "column kernel (16-cell wide columns) with 2..64 cell planes per work item"},
         "gpu_launches": mixed["launches"],
         "gpu_launches_per_step": mixed["launches"] // max(args.steps, 1),
         "fused_step": mixed["fused_step"],

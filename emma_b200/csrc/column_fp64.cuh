@@ -7,10 +7,12 @@
 // also carried its column through z (168 registers) left room for ten warps on an SM:
 // 0.51 ms a launch at 128^3, no better than the bricks' 0.53.  Here every face of a plane
 // has a thread of its own and the marching state lives in shared memory: 16 x 8-cell
-// columns, 13 warps at 72 registers, two CTAs, 26 warps on an SM; 0.396 ms (one 16 x
-// 16-cell CTA of 25 warps: 0.393 ms, but 0.030 against 0.023 ms at 32^3, where columns are
-// few).  Bound by issue (57% of cycles) and the barriers between the two phases;
-// FP64 instructions are 45% of all.  64^3: 0.072 ms (bricks 0.084); 32^3: 0.023 (0.041).
+// columns, 13 warps at 72 registers, two CTAs, 26 warps on an SM; 0.371 ms, 0.388 a step
+// with the time step's maximum (one 16 x 16-cell CTA of 25 warps: as fast there, but 0.030
+// against 0.023 ms at 32^3, where columns are few).  The 72 registers spill: 24 bytes
+// stored a thread, with gravity 88, dual energy 72, the tracer 236.  Bound by issue (57% of
+// cycles) and the barriers between the two phases; FP64 instructions are 45% of all.
+// 64^3: 0.067 ms (bricks 0.081); 32^3: 0.022 (0.041).
 //
 // Step z, two barriers:
 //   A  warps 0-5 reconstruct plane z (128 column cells, 48 ring cells) and write each

@@ -178,13 +178,15 @@ __device__ __forceinline__ void column_segments(const ColumnArgs &a, const F &se
   }
 }
 
-// FP32 reconstruction and fluxes, FP64 update; 320 threads at 96 registers, two CTAs per SM.
-// Bound by instruction issue (53% of cycles at 128^3, 17 warps an SM: 42.6 warp
-// instructions a cell, FP32 pipe 40% of them, minima, compares and selects 31%), not by
-// memory (70 bytes a cell of DRAM traffic).  Measured a launch, against slopes and all
-// three axes through shared memory and the brick kernel: 256^3 0.975 ms (1.20, 1.66), 128^3
-// 0.139 ms (0.174, 0.224); against the brick kernel, dual energy 0.159 ms (0.248) at
-// 128^3, 64^3 with transmissive x 0.031 ms (0.044).
+// FP32 reconstruction and fluxes, FP64 update; 320 threads at 96 registers (dual energy
+// spills 64 bytes, the tracer 28, gravity 8), two CTAs per SM.  Bound by instruction issue
+// (57% of cycles at 128^3, 64% at 256^3, 17 and 19 warps an SM: 42.0 warp instructions a
+// cell, FP32 pipe 41% of them, minima, compares and selects 31%), not by memory (68 and 81
+// bytes a cell of DRAM traffic).  Measured a launch without the time step's maximum,
+// against slopes and all three axes through shared memory and the brick kernel: 256^3 0.973
+// ms (1.20, 1.66), 128^3 0.139 ms (0.174, 0.223); against the brick kernel, dual energy
+// 0.160 ms (0.246) at 128^3, 64^3 with transmissive x 0.030 ms (0.043).  A step of the
+// device schedule, with the maximum: 1.038 and 0.155 ms, dual energy 0.174.
 template <bool XS, bool GRAV, bool DUAL, int NTR>
 __global__ void __launch_bounds__((Col32<DUAL, NTR>::kThreads), column_ctas(false)) column_kernel(const ColumnArgs a) {
   using M = MathF32;

@@ -29,7 +29,7 @@ def main():
     ap.add_argument("--dropin", default=None, choices=["plain", "rh"])
     ap.add_argument("--tracer", action="store_true", help="resident run of the -DWRADHYD library (dX = d/2)")
     ap.add_argument("--column", type=int, default=0,
-                    help="column kernel of complete periodic levels (mixed): 0 autotuned, -1 off, n planes per item")
+                    help="column kernel of complete levels without split cells: 0 autotuned, -1 off, n planes per item")
     ap.add_argument("--graph", action="store_true", help="also time coarse steps on the CUDA graph")
     ap.add_argument("--fused", default="auto", choices=["auto", "on", "off", "2", "3", "4"],
                     help="subcycled graph steps: autotuned, fused kernel (as many tile groups as fit, or k), "
